@@ -157,3 +157,30 @@ def test_fused_forward_with_nested_absmax(cuda):
     m_sizes = random_m_sizes(rng, M, E, 0.1)
     y = grouped_gemm_forward_4bit(to_dev(x, "bf16", cuda), packed, nested, torch.from_numpy(m_sizes).to(cuda), fused=True)
     assert_close(to_np(y), O.grouped_gemm_fwd(x, w_deq, m_sizes, "bf16"), "bf16", "nested nf4 fwd")
+
+
+@pytest.mark.parametrize("transposed", [False, True])
+@pytest.mark.parametrize("rows_per_expert", [9, 32, 300])
+def test_every_launch_decodes_the_same_weights(cuda, transposed, rows_per_expert):
+    """Decode and loads run beside each other, in an order that varies from launch to launch (the codes come from memory,
+    not from the cache: 64 experts of 1.5 MB): a decode group that read a stage before its codes had landed would change
+    some tile of some launch.  Every launch gives the same bits, those of decoding the weight first."""
+    from qwen3_moe_fused import _lib
+    from qwen3_moe_fused.grouped_gemm.forward import grouped_gemm_forward
+    from qwen3_moe_fused.grouped_gemm.forward_4bit import grouped_gemm_forward_4bit, grouped_gemm_forward_transposed_4bit
+    from qwen3_moe_fused.grouped_gemm.forward_transposed import grouped_gemm_forward_transposed
+    from qwen3_moe_fused.quantize.nf4 import dequantize_4bit, quantize_nf4
+
+    E, N, K = 64, 1536, 2048
+    torch.manual_seed(rows_per_expert)
+    packed, state = quantize_nf4(torch.randn(E, N, K, device=cuda, dtype=torch.bfloat16) * 0.02, 64)
+    ms = random_m_sizes(np.random.default_rng(rows_per_expert), rows_per_expert * E, E, 0.1)
+    m_sizes = torch.from_numpy(ms).to(cuda)
+    x = torch.randn(int(ms.sum()), N if transposed else K, device=cuda, dtype=torch.bfloat16)
+    w = dequantize_4bit(packed, state, torch.bfloat16)
+    ref = (grouped_gemm_forward_transposed if transposed else grouped_gemm_forward)(x, w, m_sizes)
+    for i in range(100):
+        y = grouped_gemm_forward_transposed_4bit(x, packed, state, m_sizes) if transposed else \
+            grouped_gemm_forward_4bit(x, packed, state, m_sizes, fused=True)
+        assert torch.equal(y, ref), f"launch {i}"
+    assert _lib.read_error_flag() == 0

@@ -4,8 +4,8 @@
 // Same tiling as pair_fwd_kernel<false> (accumulator rows = 256 weight rows of one expert,
 // 128 per CTA; accumulator columns = up to 256 tokens; two TMEM accumulators so the epilogue
 // overlaps the next tile), but the weight half-tile of a stage is not loaded as 16-bit data:
-// TMA brings the 4 KB of packed 4-bit codes (128 rows x 32 bytes) and sixteen decode warps per
-// CTA (four groups of four, taking k-blocks in turn) expand them to the swizzled K-major 16-bit tile the MMA reads.  HBM and L2 see
+// TMA brings the 4 KB of packed 4-bit codes (128 rows x 32 bytes) and twenty decode warps per
+// CTA (five groups of four, taking k-blocks in turn) expand them to the swizzled K-major 16-bit tile the MMA reads.  HBM and L2 see
 // 0.5 + 4/blocksize bytes per weight instead of 2.
 //
 // Synchronisation per stage s:
@@ -35,12 +35,14 @@
 namespace moe {
 namespace tc {
 
-#ifndef MOE_NF4P_GROUPS
-#define MOE_NF4P_GROUPS 4
-#endif
-constexpr int NF4P_GROUPS = MOE_NF4P_GROUPS;                    // decode groups of four warps, taking k-blocks in turn
-constexpr int NF4P_THREADS = 192 + NF4P_GROUPS * 128;           // TMA, MMA, 4 epilogue warps + the decode warps
 constexpr int NF4P_STAGES = 5;
+constexpr int NF4P_GROUPS = 5;                                  // decode groups of four warps, taking k-blocks in turn
+constexpr int NF4P_THREADS = 192 + NF4P_GROUPS * 128;           // TMA, MMA, 4 epilogue warps + the decode warps
+// A decode group must meet the phases of a stage's qfull barrier one after the other.  If it came back to a
+// stage after skipping a phase (say 4 groups on 5 stages: k-block j, then j + 4 in the stage of j - 1), it
+// could test for the phase of j + 4 while the codes of j - 1 were still on their way (loads complete in any
+// order); the parity of that phase equals the one before j - 1, so the test would pass at once.
+static_assert(NF4P_STAGES % NF4P_GROUPS == 0, "every stage belongs to one decode group");
 constexpr int NF4P_PACKED_BYTES = 128 * (BK / 2);               // 4 KB
 constexpr int NF4P_STAGE_BYTES = 2 * PAIR_HALF_BYTES + NF4P_PACKED_BYTES;  // 36 KB
 
@@ -278,7 +280,7 @@ pair_fwd_nf4_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
     // ------------------------------ decode warps (both CTAs) ------------------------------
     // NF4P_GROUPS groups of four warps take the k-blocks in turn, so the decode of one k-block (a
     // few hundred cycles of dependent work per thread) overlaps the decode of the next ones.
-    // Measured at 262144 rows: 2 groups 1162 TFLOP/s, 4 groups 1255.  Inside a
+    // Measured at 262144 rows: 2 groups 1162 TFLOP/s, 4 groups 1255 (5: see the static_assert above).  Inside a
     // group, thread -> weight row (t % 128) of this CTA's half-tile; it decodes the row's 64
     // weights of the k-block (32 packed bytes, one absmax).
     const int t = threadIdx.x - 6 * 32;
@@ -340,7 +342,7 @@ pair_fwd_nf4_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
         }
         fence_proxy_async_smem();
         __syncwarp();
-        if (lane == 0) mbar_arrive_cluster(ready_leader0 + s * 8);
+        if (lane == 0) mbar_arrive_release_cluster(ready_leader0 + s * 8);
       }
       it += k_blocks;
     }
