@@ -221,6 +221,12 @@ int moe_router_softmax_topk(const void* logits, int dtype_logits, int64_t T, int
                             int norm_topk, void* weights, int dtype_w, int64_t* experts,
                             void* stream);
 
+/* Gradient of the logits from the gradient of moe_router_softmax_topk's weights (dtype_w); `experts` as
+ * that call returned them.  dlogits has the dtype of the logits.
+ * Replaces the autograd of qwen3_moe_fused/modular_qwen3_moe_fused.py:87-93. */
+int moe_router_softmax_topk_bwd(const void* logits, int dtype_logits, const int64_t* experts, const void* dweights,
+                                int dtype_w, int64_t T, int E, int k, int norm_topk, void* dlogits, void* stream);
+
 /* out[j,:] = hidden[sort_idx[j] / k, :]   (expand by k then gather, in one pass).
  * Replaces qwen3_moe_fused/modular_qwen3_moe_fused.py:95-103. */
 int moe_gather_rows(const void* hidden, const int32_t* sort_idx, int k, void* out,
@@ -237,6 +243,13 @@ int moe_expand_rows(const void* hidden, const int32_t* inv_sort_idx, int k, void
  * Replaces qwen3_moe_fused/modular_qwen3_moe_fused.py:112-115. */
 int moe_combine(const void* y, const int32_t* inv_sort_idx, const void* weights, void* out,
                 int64_t T, int k, int H, int dtype, void* stream);
+
+/* Backward of moe_combine in one pass: dy[inv_sort_idx[t*k+j], :] = weights[t,j] * dout[t,:] and
+ * dweights[t,j] = <dout[t,:], y[inv_sort_idx[t*k+j], :]> (fp32 sums).  dy or dweights may be NULL (not wanted);
+ * weights is read for dy, y for dweights.
+ * Replaces the autograd of qwen3_moe_fused/modular_qwen3_moe_fused.py:110-115. */
+int moe_combine_bwd(const void* dout, const void* y, const int32_t* inv_sort_idx, const void* weights, void* dy,
+                    void* dweights, int64_t T, int k, int H, int dtype, void* stream);
 
 /* ---------------------------------------------------------------------------------
  * Expert parallelism over peer memory.  The reference has no multi-GPU path

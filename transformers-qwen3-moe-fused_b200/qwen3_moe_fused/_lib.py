@@ -48,9 +48,11 @@ SIGNATURES = {
     "moe_silu_mul_bwd": (_I, [_P, _P, _P, _P, _P, _L, _I, _P]),
     "moe_silu_mul_bwd_inplace": (_I, [_P, _P, _P, _L, _I, _P]),
     "moe_router_softmax_topk": (_I, [_P, _I, _L, _I, _I, _I, _P, _I, _P, _P]),
+    "moe_router_softmax_topk_bwd": (_I, [_P, _I, _P, _P, _I, _L, _I, _I, _I, _P, _P]),
     "moe_gather_rows": (_I, [_P, _P, _I, _P, _L, _I, _I, _P]),
     "moe_expand_rows": (_I, [_P, _P, _I, _P, _L, _I, _I, _P]),
     "moe_combine": (_I, [_P, _P, _P, _P, _L, _I, _I, _I, _P]),
+    "moe_combine_bwd": (_I, [_P, _P, _P, _P, _P, _P, _L, _I, _I, _I, _P]),
     "moe_ep_plan": (_I, [_P, _I, _I, _I, _I, _I, _P, _P, _P, _P, _P, _P, _P, _P, _P]),
     "moe_ep_push_rows": (_I, [_P, _L, _L, _P, _I, _I, _P, _P, _I, _P, _I, _I, _P, _P]),
     "moe_ep_token_positions": (_I, [_P, _I, _L, _I, _I, _I, _P, _P, _P]),

@@ -27,28 +27,31 @@ def softmax_topk(router_logits: torch.Tensor, k: int, norm_topk_prob: bool, out_
 
 
 class SoftmaxTopk(torch.autograd.Function):
-    """Differentiable wrapper: the forward is one kernel; the backward recomputes the fp32
-    softmax of the (T, E) logits and differentiates gather -> renormalise -> cast, which is
-    what autograd does for the reference's sequence of ATen calls."""
+    """Differentiable wrapper: the forward is one kernel; the backward is one kernel that
+    recomputes the fp32 softmax of the (T, E) logits and differentiates gather -> renormalise
+    -> cast, which is what autograd does for the reference's sequence of ATen calls."""
 
     @staticmethod
     def forward(ctx, router_logits, k, norm_topk_prob, out_dtype):
         weights, experts = softmax_topk(router_logits, k, norm_topk_prob, out_dtype)
         ctx.save_for_backward(router_logits, experts)
         ctx.norm = norm_topk_prob
-        ctx.out_dtype = out_dtype
         ctx.mark_non_differentiable(experts)
         return weights, experts
 
     @staticmethod
     def backward(ctx, dweights, _dexperts):
         logits, experts = ctx.saved_tensors
-        with torch.enable_grad():
-            lg = logits.detach().requires_grad_()
-            sel = torch.softmax(lg, dim=1, dtype=torch.float32).gather(1, experts)
-            if ctx.norm:
-                sel = sel / sel.sum(dim=-1, keepdim=True)
-            (grad,) = torch.autograd.grad(sel.to(ctx.out_dtype), lg, dweights)
+        T, E = logits.shape
+        dweights = dweights.contiguous()
+        grad = torch.empty_like(logits)
+        with torch.cuda.device(logits.device):
+            status = _lib.load().moe_router_softmax_topk_bwd(
+                _lib.ptr(logits), _lib.float_code(logits.dtype), _lib.ptr(experts), _lib.ptr(dweights),
+                _lib.float_code(dweights.dtype), T, E, experts.shape[1], int(ctx.norm), _lib.ptr(grad),
+                _lib.stream_ptr(logits.device),
+            )
+        _lib.check(status, "moe_router_softmax_topk_bwd")
         return grad, None, None, None
 
 
@@ -137,11 +140,15 @@ class Combine(torch.autograd.Function):
         dout = dout.contiguous()
         dy = dw = None
         if ctx.needs_input_grad[0]:
-            # dy[j] = weights.flat[sort_idx[j]] * dout[sort_idx[j] // k]
-            dy = _expand_rows(dout, inv_sort_idx, k) * weights.reshape(-1)[sort_idx.long()].unsqueeze(1)
+            dy = torch.empty((T * k, y.shape[1]), device=y.device, dtype=y.dtype)
         if ctx.needs_input_grad[3]:
-            # dweights[t, j] = <dout[t], y[inv_sort_idx[t*k+j]]>
-            dw = torch.einsum("tkh,th->tk", y[inv_sort_idx.long()].view(T, k, -1).float(), dout.float()).to(weights.dtype)
+            dw = torch.empty((T, k), device=y.device, dtype=weights.dtype)
+        with torch.cuda.device(y.device):
+            status = _lib.load().moe_combine_bwd(
+                _lib.ptr(dout), _lib.ptr(y), _lib.ptr(inv_sort_idx), _lib.ptr(weights), _lib.ptr(dy), _lib.ptr(dw),
+                T, k, y.shape[1], _lib.float_code(y.dtype), _lib.stream_ptr(y.device),
+            )
+        _lib.check(status, "moe_combine_bwd")
         return dy, None, None, dw
 
 
