@@ -167,7 +167,8 @@ dw_kernel(const __grid_constant__ CUtensorMap tmap_out, const GemmParams p) {
       // at one item later, so that the atomic's round trip overlaps the loads in between)
       uint32_t drawn = 0;
       auto draw = [&]() -> int64_t {
-        const int64_t t = p.tile_counter ? (int64_t)atomicAdd(p.tile_counter, 1) : (int64_t)unit + (int64_t)drawn * G;
+        const int64_t t = drawn == 0 ? (int64_t)unit : p.tile_counter ? (int64_t)atomicAdd(p.tile_counter, 1) + G
+                                                                      : (int64_t)unit + (int64_t)drawn * G;
         ++drawn;
         return t;
       };
