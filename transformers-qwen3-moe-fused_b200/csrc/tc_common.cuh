@@ -232,6 +232,25 @@ __device__ __forceinline__ void tma_load_3d_pair(void* smem_dst, const CUtensorM
       ::"r"(smem_u32(smem_dst)), "l"((uint64_t)map), "r"(bar_cluster_addr), "r"(x), "r"(y), "r"(z)
       : "memory");
 }
+// Cluster launch control: asks for a cluster of this grid that has not started yet; if there is one it will not
+// start, and the caller does its work.  16 bytes arrive at `response` and complete on `bar`.  One request at a
+// time, and none after one that found no cluster.  Not multicast: the answer goes to the issuing CTA only.
+__device__ __forceinline__ void cluster_try_cancel(void* response, uint64_t* bar) {
+  asm volatile("clusterlaunchcontrol.try_cancel.async.shared::cta.mbarrier::complete_tx::bytes.b128 [%0], [%1];"
+               ::"r"(smem_u32(response)), "r"(smem_u32(bar)) : "memory");
+}
+// blockIdx.x of the cancelled cluster's first CTA, or -1 if no cluster was left.
+__device__ __forceinline__ int cluster_cancelled_cta(const void* response) {
+  int x;
+  asm volatile(
+      "{\n\t.reg .b128 r;\n\t.reg .b64 lo, hi;\n\t.reg .pred p;\n\t"
+      "ld.shared.v2.b64 {lo, hi}, [%1];\n\tmov.b128 r, {lo, hi};\n\t"
+      "mov.b32 %0, -1;\n\t"
+      "clusterlaunchcontrol.query_cancel.is_canceled.pred.b128 p, r;\n\t"
+      "@p clusterlaunchcontrol.query_cancel.get_first_ctaid::x.b32.b128 %0, r;\n\t}"
+      : "=&r"(x) : "r"(smem_u32(response)) : "memory");
+  return x;
+}
 // Four rows of a 2-D tensor, given by their row indices, into four consecutive 128-byte rows of shared
 // memory (the tensor map's box is {64 elements, 1 row}); completion as for the loads above.  Rows whose
 // index lies outside the tensor are filled with zeros.  Not multicast.

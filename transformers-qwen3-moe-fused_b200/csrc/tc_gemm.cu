@@ -40,11 +40,11 @@ struct GemmParams {
   int ms64;
   int dtype_out;  // MOE_F32 / MOE_BF16 / MOE_F16
   uint32_t idesc;
-  const CUtensorMap* group_maps;  // per-expert tensor maps in workspace ([slot][expert]), or null
+  const CUtensorMap* group_maps = nullptr;  // per-expert tensor maps in workspace ([slot][expert]), or null
   const int* weight_index = nullptr;  // weight slice of each group (null: group e uses slice e)
   int* tile_counter = nullptr;  // work items are drawn from this counter (zeroed by build_group_maps_kernel); null: round-robin
   int stages = 0;               // CTA-pair forward / dX: depth of the operand ring
-  int small_maps = 0;           // CTA-pair forward / dX: per-expert maps with the small token box exist (slot GM_IN_SMALL)
+  int staged = 0;               // CTA-pair forward / dX: 16-bit output that may leave by TMA
   const int* row_index = nullptr;  // gathered forms: sorted row r reads row row_index[r] / index_div of the token tensor
   int index_div = 1;
   int64_t x_rows = 0;           // gathered forms: rows of the token tensor
@@ -582,17 +582,18 @@ static EncodeTiledFn encode_fn() {
 }
 
 // Tensor map over a dense 16-bit tensor viewed as (d2, d1, d0) with d0 contiguous.
-// Box = (b0 = 64 elements, b1 rows, 1).  rank 2 when d2 == 0.
+// Box = (b0 = 64 elements, b1 rows, 1).  rank 2 when d2 == 0.  `pitch`: elements between rows (0: d0).
 thread_local char g_detail[320] = "";
 
 static int make_map(CUtensorMap* map, int dtype, const void* base, uint64_t d0, uint64_t d1, uint64_t d2,
-                    uint32_t b1) {
+                    uint32_t b1, uint64_t pitch = 0) {
   EncodeTiledFn fn = encode_fn();
   if (!fn) return MOE_ERR_DEVICE;
   const CUtensorMapDataType dt = dtype == MOE_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16;
   const cuuint32_t rank = d2 ? 3 : 2;
   cuuint64_t dims[3] = {d0, d1, d2 ? d2 : 1};
-  cuuint64_t strides[2] = {d0 * 2, d0 * d1 * 2};
+  if (pitch == 0) pitch = d0;
+  cuuint64_t strides[2] = {pitch * 2, pitch * d1 * 2};
   cuuint32_t box[3] = {64, b1, 1};
   cuuint32_t estr[3] = {1, 1, 1};
   const CUresult r = fn(map, dt, rank, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
@@ -734,92 +735,100 @@ static int pair_stages(int E) {
   return 0;
 }
 
-// Launches build_group_maps_kernel for the forward / dX / gate-up kernels: per-expert copies of the
-// token maps (128-row and small box) and, for 16-bit outputs, of the output map.
-static int build_pair_maps(tc::GemmParams& p, const CUtensorMap& mx, const void* a, void* out, int dtype_in, int dtype_out,
-                           void* ws, cudaStream_t stream, const uint64_t* out_ptrs, bool gather = false) {
+// Clusters to launch: no fewer than there are tiles (every group of r rows has at most r / 256 + 1 token tiles).
+static int64_t pair_tiles_bound(int64_t M, int E, int n_tiles) {
+  return (M / tc::PAIR_TOKENS + (M < E ? M : E)) * n_tiles;
+}
+
+// One activation tensor and the weights it is contracted with: x (M rows of K, `pitch` elements apart), w (E, N, K)
+// or, for dX, (E, K, N).
+struct PairOperand {
+  const void* x;
+  const void* w;
+  int K;
+  int64_t pitch;
+};
+
+static int fill_pair_operand(tc::PairMaps& maps, int i, int which, const PairOperand& o, int64_t M, int N, int n_weights,
+                             int dtype_in) {
   using namespace tc;
-  GroupMapTemplates tm;
   int st;
-  tm.mask = 0;
-  if (!gather) {  // (gathered token rows are addressed by index: no per-expert token maps)
-    tm.mask = (1 << GM_IN) | (1 << GM_IN_SMALL);
-    tm.t[GM_IN] = mx;
-    if ((st = make_map(&tm.t[GM_IN_SMALL], dtype_in, a, (uint64_t)p.K, (uint64_t)p.M, 0, PAIR_SMALL_BOX)) != MOE_OK) return st;
-  }
-  if (dtype_out != MOE_F32) {
-    tm.mask |= 1 << GM_OUT;
-    if ((st = make_map(&tm.t[GM_OUT], dtype_out, out, (uint64_t)p.N, (uint64_t)p.M, 0, 32)) != MOE_OK) return st;
-  }
-  const int gm_smem = 8 * 128 + 2 * (p.E + 1) * 4 + 128;
-  build_group_maps_kernel<<<(p.E + 7) / 8, 256, gm_smem, stream>>>(tm, p.m_sizes, p.ms64, p.E, p.M, reinterpret_cast<CUtensorMap*>(ws),
-                                                                   ws_counter(ws, p.E), out_ptrs, GM_OUT, (int64_t)p.N * 2);
-  if ((st = launch_status()) != MOE_OK) return st;
-  p.group_maps = reinterpret_cast<const CUtensorMap*>(ws);
-  p.tile_counter = ws_counter(ws, p.E);
-  p.small_maps = gather ? 0 : 1;
+  // A = weight (accumulator rows), B = activations (accumulator columns = tokens)
+  if (which == 0) st = make_map(&maps.w[i], dtype_in, o.w, (uint64_t)o.K, (uint64_t)N, (uint64_t)n_weights, 128);
+  else st = make_map(&maps.w[i], dtype_in, o.w, (uint64_t)N, (uint64_t)o.K, (uint64_t)n_weights, BK);
+  if (st != MOE_OK) return st;
+  if ((st = make_map(&maps.x[i], dtype_in, o.x, (uint64_t)o.K, (uint64_t)M, 0, 128, (uint64_t)o.pitch)) != MOE_OK) return st;
+  if ((st = make_map(&maps.xs[i], dtype_in, o.x, (uint64_t)o.K, (uint64_t)M, 0, PAIR_SMALL_BOX, (uint64_t)o.pitch)) != MOE_OK) return st;
+  maps.kb[i] = (o.K + BK - 1) / BK;
+  maps.last_steps[i] = (o.K - (maps.kb[i] - 1) * BK + UMMA_K - 1) / UMMA_K;
   return MOE_OK;
+}
+
+template <typename Kern>
+static int launch_pair_fwd(Kern kern, const tc::PairMaps& maps, tc::GemmParams& p, int n_tiles, cudaStream_t stream) {
+  using namespace tc;
+  p.stages = pair_stages(p.E);
+  if (p.stages == 0) return MOE_ERR_UNSUPPORTED;
+  const int bytes = pair_smem_bytes(p.stages, p.E);
+  int st;
+  if ((st = set_smem(kern, bytes)) != MOE_OK) return st;
+  kern<<<(unsigned)(2 * pair_tiles_bound(p.M, p.E, n_tiles)), PAIR_THREADS, bytes, stream>>>(maps, p);
+  return launch_status();
 }
 
 // `weight_index` / `n_weights` / `out_ptrs` (all optional) describe the scattered form: group e
 // multiplies by weight slice weight_index[e] of n_weights, and its output rows start at the
 // address out_ptrs[e] instead of row row_start[e] of `out`.
-static int pair_grouped_gemm(int which, const void* a, const void* b, const void* m_sizes, int ms64, void* out,
-                             int64_t M, int N, int K, int E, int dtype_in, int dtype_out, void* ws, size_t ws_bytes,
+static int pair_grouped_gemm(int which, const PairOperand* ops, int n_ops, const void* m_sizes, int ms64, void* out,
+                             int64_t M, int N, int E, int dtype_in, int dtype_out, void* ws, size_t ws_bytes,
                              cudaStream_t stream, const int* weight_index = nullptr, int n_weights = 0,
                              const uint64_t* out_ptrs = nullptr, const int* row_index = nullptr, int index_div = 1,
                              int64_t x_rows = 0) {
   using namespace tc;
-  if (which != 0 && which != 1) return MOE_ERR_UNSUPPORTED;
+  if ((which != 0 && which != 1) || n_ops < 1 || n_ops > PAIR_MAX_SEGS) return MOE_ERR_UNSUPPORTED;
   const bool gather = row_index != nullptr;
-  if (gather && (which != 0 || index_div <= 0 || x_rows <= 0 || x_rows > 0x7fffffffLL)) return MOE_ERR_UNSUPPORTED;
+  if (gather && (which != 0 || n_ops != 1 || index_div <= 0 || x_rows <= 0 || x_rows > 0x7fffffffLL)) return MOE_ERR_UNSUPPORTED;
   if (n_weights <= 0) n_weights = E;
   GemmParams p;
   p.row_index = row_index; p.index_div = index_div; p.x_rows = x_rows;
   p.weight_index = weight_index;
-  p.a = a; p.b = b;
-  p.m_sizes = m_sizes; p.out = out; p.M = M; p.N = N; p.K = K; p.E = E; p.ms64 = ms64; p.dtype_out = dtype_out;
-  const int fmt = dtype_in == MOE_BF16 ? 1 : 0;
-  p.group_maps = nullptr;
+  p.a = ops[0].x; p.b = ops[0].w;
+  p.m_sizes = m_sizes; p.out = out; p.M = M; p.N = N; p.K = ops[0].K; p.E = E; p.ms64 = ms64; p.dtype_out = dtype_out;
+  const int n_tiles = (N + 255) / 256;
   // tile ids are 32-bit
-  if (((M + PAIR_TOKENS - 1) / PAIR_TOKENS + E) * (int64_t)((N + 255) / 256) >= (int64_t)1 << 30) return MOE_ERR_UNSUPPORTED;
-  CUtensorMap mw, mx;
+  if (((M + PAIR_TOKENS - 1) / PAIR_TOKENS + E) * (int64_t)n_tiles >= (int64_t)1 << 30) return MOE_ERR_UNSUPPORTED;
+  PairMaps maps;
+  memset(&maps, 0, sizeof(maps));
+  maps.n_seg = n_ops;
   int st;
-  // A = weight (accumulator rows), B = activations (accumulator columns = tokens)
-  if (which == 0) st = make_map(&mw, dtype_in, b, (uint64_t)K, (uint64_t)N, (uint64_t)n_weights, 128);
-  else st = make_map(&mw, dtype_in, b, (uint64_t)N, (uint64_t)K, (uint64_t)n_weights, BK);
-  if (st != MOE_OK) return st;
-  // token map: 128-row boxes over the M sorted rows, or one-row boxes (for gather4) over the x_rows token rows
-  if (gather) st = make_map(&mx, dtype_in, a, (uint64_t)K, (uint64_t)x_rows, 0, 1);
-  else st = make_map(&mx, dtype_in, a, (uint64_t)K, (uint64_t)M, 0, 128);
-  if (st != MOE_OK) return st;
-  p.idesc = make_idesc(fmt, which == 1, 0, 256, 0);  // N field is filled per tile
-  // Per-expert copies of the token and output maps (row extent = the group's last row): partial
-  // tiles then load no rows of the next expert, and 16-bit outputs can leave through TMA stores.
-  if (ws_usable(ws, ws_bytes, E) && (((uintptr_t)out & 15) == 0 || dtype_out == MOE_F32)) {
-    if ((st = build_pair_maps(p, mx, a, out, dtype_in, dtype_out, ws, stream, out_ptrs, gather)) != MOE_OK) return st;
+  for (int i = 0; i < n_ops; ++i)
+    if ((st = fill_pair_operand(maps, i, which, ops[i], gather ? x_rows : M, N, n_weights, dtype_in)) != MOE_OK) return st;
+  // gathered token rows: one-row boxes (for gather4) over the x_rows token rows
+  if (gather && (st = make_map(&maps.x[0], dtype_in, ops[0].x, (uint64_t)ops[0].K, (uint64_t)x_rows, 0, 1)) != MOE_OK) return st;
+  p.idesc = make_idesc(dtype_in == MOE_BF16 ? 1 : 0, which == 1, 0, 256, 0);  // N field is filled per tile
+  const bool out_ok = ((uintptr_t)out & 15) == 0 || dtype_out == MOE_F32;
+  if (gather && !(ws_usable(ws, ws_bytes, E) && out_ok)) return MOE_ERR_WORKSPACE;
+  p.staged = out_ok && dtype_out != MOE_F32;
+  if (p.staged && (st = make_map(&maps.out, dtype_out, out, (uint64_t)N, (uint64_t)M, 0, 32)) != MOE_OK) return st;
+  if (out_ptrs != nullptr) {
+    // scattered outputs: one output map per group, re-based on its address and clipped at its last row
+    if (!p.staged || !ws_usable(ws, ws_bytes, E)) return MOE_ERR_UNSUPPORTED;
+    GroupMapTemplates tm;
+    tm.mask = 1 << GM_OUT;
+    tm.t[GM_OUT] = maps.out;
+    const int gm_smem = 8 * 128 + 2 * (E + 1) * 4 + 128;
+    build_group_maps_kernel<<<(E + 7) / 8, 256, gm_smem, stream>>>(tm, m_sizes, ms64, E, M, reinterpret_cast<CUtensorMap*>(ws),
+                                                                   nullptr, out_ptrs, GM_OUT, (int64_t)N * 2);
+    if ((st = launch_status()) != MOE_OK) return st;
+    p.group_maps = reinterpret_cast<const CUtensorMap*>(ws);
   }
-  if (gather && p.group_maps == nullptr) return MOE_ERR_WORKSPACE;
-  // scattered outputs exist only as per-group output maps
-  if (out_ptrs != nullptr && (p.group_maps == nullptr || dtype_out == MOE_F32)) return MOE_ERR_UNSUPPORTED;
-  p.stages = pair_stages(E);
-  if (p.stages == 0) return MOE_ERR_UNSUPPORTED;
-  const int bytes = pair_smem_bytes(p.stages, E);
-  if (gather) {
-    auto kern = pair_fwd_kernel<false, false, true>;
-    if ((st = set_smem(kern, bytes)) != MOE_OK) return st;
-    const int grid = 2 * resident_pairs(kern, bytes);
-    kern<<<grid, PAIR_THREADS, bytes, stream>>>(mw, mx, p, mw);
-  } else if (which == 0) {
-    if ((st = set_smem(pair_fwd_kernel<false>, bytes)) != MOE_OK) return st;
-    const int grid = 2 * resident_pairs(pair_fwd_kernel<false>, bytes);
-    pair_fwd_kernel<false><<<grid, PAIR_THREADS, bytes, stream>>>(mw, mx, p, mw);
-  } else {
-    if ((st = set_smem(pair_fwd_kernel<true>, bytes)) != MOE_OK) return st;
-    const int grid = 2 * resident_pairs(pair_fwd_kernel<true>, bytes);
-    pair_fwd_kernel<true><<<grid, PAIR_THREADS, bytes, stream>>>(mw, mx, p, mw);
+  if (gather) return launch_pair_fwd(pair_fwd_kernel<false, false, true>, maps, p, n_tiles, stream);
+  if (n_ops > 1) {
+    if (which == 0) return launch_pair_fwd(pair_fwd_kernel<false, false, false, true>, maps, p, n_tiles, stream);
+    return launch_pair_fwd(pair_fwd_kernel<true, false, false, true>, maps, p, n_tiles, stream);
   }
-  return launch_status();
+  if (which == 0) return launch_pair_fwd(pair_fwd_kernel<false>, maps, p, n_tiles, stream);
+  return launch_pair_fwd(pair_fwd_kernel<true>, maps, p, n_tiles, stream);
 }
 
 // Launch with a cluster of 2 CTAs.
@@ -920,7 +929,8 @@ int tc_grouped_gemm(int which, const void* a, const void* b, const void* m_sizes
     // a pair covers 256 weight rows (and, for dW, 256 weight columns): narrower problems
     // would leave most of the tile empty
     const bool pair_ok = N >= 192;
-    if (pair_ok) return pair_grouped_gemm(which, a, b, m_sizes, ms64, out, M, N, K, E, dtype_in, dtype_out, ws, ws_bytes, stream);
+    const PairOperand op{a, b, K, 0};
+    if (pair_ok) return pair_grouped_gemm(which, &op, 1, m_sizes, ms64, out, M, N, E, dtype_in, dtype_out, ws, ws_bytes, stream);
   }
   GemmParams p;
   p.m_sizes = m_sizes; p.out = out; p.M = M; p.N = N; p.K = K; p.E = E; p.ms64 = ms64; p.dtype_out = dtype_out;
@@ -978,31 +988,25 @@ int tc_gate_up_silu(const void* x, const void* w_gate, const void* w_up, const v
   p.m_sizes = m_sizes; p.out = h; p.M = M; p.N = I; p.K = K; p.E = E; p.ms64 = ms64; p.dtype_out = dtype;
   p.idesc = make_idesc(dtype == MOE_BF16 ? 1 : 0, 0, 0, 256, 0);
   if (((M + PAIR_TOKENS - 1) / PAIR_TOKENS + E) * (int64_t)((I + 127) / 128) >= (int64_t)1 << 30) return MOE_ERR_UNSUPPORTED;
-  CUtensorMap mg, mu, mx;
+  PairMaps maps;
+  memset(&maps, 0, sizeof(maps));
+  maps.n_seg = 1;
   int st;
-  if ((st = make_map(&mg, dtype, w_gate, (uint64_t)K, (uint64_t)I, (uint64_t)E, 16)) != MOE_OK) return st;
-  if ((st = make_map(&mu, dtype, w_up, (uint64_t)K, (uint64_t)I, (uint64_t)E, 16)) != MOE_OK) return st;
+  if ((st = make_map(&maps.w[0], dtype, w_gate, (uint64_t)K, (uint64_t)I, (uint64_t)E, 16)) != MOE_OK) return st;
+  if ((st = make_map(&maps.w[1], dtype, w_up, (uint64_t)K, (uint64_t)I, (uint64_t)E, 16)) != MOE_OK) return st;
   const bool gather = row_index != nullptr;
   if (gather && (index_div <= 0 || x_rows <= 0 || x_rows > 0x7fffffffLL)) return MOE_ERR_SHAPE;
   p.row_index = row_index; p.index_div = index_div; p.x_rows = x_rows;
-  if (gather) st = make_map(&mx, dtype, x, (uint64_t)K, (uint64_t)x_rows, 0, 1);
-  else st = make_map(&mx, dtype, x, (uint64_t)K, (uint64_t)M, 0, 128);
+  if (gather) st = make_map(&maps.x[0], dtype, x, (uint64_t)K, (uint64_t)x_rows, 0, 1);
+  else st = make_map(&maps.x[0], dtype, x, (uint64_t)K, (uint64_t)M, 0, 128);
   if (st != MOE_OK) return st;
-  if ((st = build_pair_maps(p, mx, x, h, dtype, dtype, ws, stream, nullptr, gather)) != MOE_OK) return st;
-  p.stages = pair_stages(E);
-  if (p.stages == 0) return MOE_ERR_UNSUPPORTED;
-  const int bytes = pair_smem_bytes(p.stages, E);
-  if (gather) {
-    auto kern = pair_fwd_kernel<false, true, true>;
-    if ((st = set_smem(kern, bytes)) != MOE_OK) return st;
-    kern<<<2 * resident_pairs(kern, bytes), PAIR_THREADS, bytes, stream>>>(mg, mx, p, mu);
-    return launch_status();
-  }
-  auto kern = pair_fwd_kernel<false, true>;
-  if ((st = set_smem(kern, bytes)) != MOE_OK) return st;
-  const int grid = 2 * resident_pairs(kern, bytes);
-  kern<<<grid, PAIR_THREADS, bytes, stream>>>(mg, mx, p, mu);
-  return launch_status();
+  if (!gather && (st = make_map(&maps.xs[0], dtype, x, (uint64_t)K, (uint64_t)M, 0, PAIR_SMALL_BOX)) != MOE_OK) return st;
+  if ((st = make_map(&maps.out, dtype, h, (uint64_t)I, (uint64_t)M, 0, 32)) != MOE_OK) return st;
+  maps.kb[0] = (K + BK - 1) / BK;
+  p.staged = 1;
+  const int n_tiles = (I + 127) / 128;
+  if (gather) return launch_pair_fwd(pair_fwd_kernel<false, true, true>, maps, p, n_tiles, stream);
+  return launch_pair_fwd(pair_fwd_kernel<false, true>, maps, p, n_tiles, stream);
 }
 
 // Forward whose sorted row r is row row_index[r] / index_div of x (x_rows rows): CTA-pair kernel only.
@@ -1011,7 +1015,8 @@ int tc_grouped_gemm_gather(const void* x, int64_t x_rows, const int* row_index, 
                            int dtype_out, void* ws, size_t ws_bytes, cudaStream_t stream) {
   bind_context_once();
   if (N < 192) return MOE_ERR_UNSUPPORTED;
-  return pair_grouped_gemm(0, x, w, m_sizes, ms64, y, M, N, K, E, dtype_in, dtype_out, ws, ws_bytes, stream, nullptr, 0,
+  const PairOperand op{x, w, K, 0};
+  return pair_grouped_gemm(0, &op, 1, m_sizes, ms64, y, M, N, E, dtype_in, dtype_out, ws, ws_bytes, stream, nullptr, 0,
                            nullptr, row_index, index_div, x_rows);
 }
 
@@ -1022,7 +1027,8 @@ int tc_grouped_gemm_scattered(int which, const void* a, const void* b, const voi
                               cudaStream_t stream) {
   bind_context_once();
   if (which != 0 && which != 1) return MOE_ERR_UNSUPPORTED;
-  return pair_grouped_gemm(which, a, b, group_sizes, ms64, out_template, M, N, K, G, dtype_in, dtype_out, ws, ws_bytes,
+  const PairOperand op{a, b, K, 0};
+  return pair_grouped_gemm(which, &op, 1, group_sizes, ms64, out_template, M, N, G, dtype_in, dtype_out, ws, ws_bytes,
                            stream, weight_index, n_weights, out_ptrs);
 }
 

@@ -29,12 +29,20 @@
 // first, so the next tile's MMAs wait for one or two 32-column rounds of the epilogue, not for
 // all of it; tiles without a tail never wait for each other.
 //
-// Tile order.  Tiles are handed out in index order from a global counter (one atomicAdd per
-// tile, by a thread that has nothing else to do: warp 1 of the non-leader CTA), and travel to
-// the working roles of both CTAs through a small ring in shared memory, several tiles ahead of
-// their use: ragged groups make tile costs uneven, and a static round-robin left a fifth of
-// the pairs idle at the end.  Without a counter (no workspace) the same ring carries a static
-// round-robin order.
+// Tile order.  The grid has one cluster per tile (an upper bound taken from M and E); a running pair takes
+// over the next cluster that has not started yet (clusterlaunchcontrol.try_cancel, by a thread that has nothing
+// else to do: warp 1 of the non-leader CTA), so the tiles are handed out in index order to whichever pair is
+// free: ragged groups make tile costs uneven, and a static round-robin left a fifth of the pairs idle at the
+// end.  The ids travel to the working roles of both CTAs through a small ring in shared memory.  (A counter in
+// global memory did the same before; it had to be zeroed by a launch of its own, 7 us with its gap per GEMM.)
+//
+// Groups and tensor maps.  The token maps cover all rows: a partial tile's last box may bring in rows of the
+// next group, whose accumulator columns are never stored.  A 32-row round of the epilogue that lies inside the
+// group leaves by TMA; the group's last round, if it is partial, is copied row by row from the staging tile.
+//
+// Segments.  The contraction may run over several (weight, activation) operand pairs into one accumulator:
+//     y[t,:] = sum_i  W_i[e] x_i[t,:]
+// (base weight + LoRA product, or gate + up gradients): see PairMaps.
 #pragma once
 
 namespace moe {
@@ -66,37 +74,66 @@ struct SchedRing {
   int tile[SCHED_DEPTH];
 };
 
+// Operands of one launch: segment i contracts w[i] with x[i] over kb[i] blocks of 64.
+constexpr int PAIR_MAX_SEGS = 4;
+struct PairMaps {
+  CUtensorMap w[PAIR_MAX_SEGS];   // weights (GATE_UP: [0] gate, [1] up)
+  CUtensorMap x[PAIR_MAX_SEGS];   // activations, 128-row boxes (GATHER: one-row boxes over the token tensor)
+  CUtensorMap xs[PAIR_MAX_SEGS];  // activations, boxes of PAIR_SMALL_BOX rows
+  CUtensorMap out;                // 16-bit outputs: boxes of 32 rows
+  int kb[PAIR_MAX_SEGS];
+  int last_steps[PAIR_MAX_SEGS];  // MMA steps of 16 in the last block (MULTI)
+  int n_seg;
+};
+
 struct PairControl {
   uint64_t full[8];
   uint64_t empty[8];
   uint64_t tmem_full[2];
   uint64_t tmem_free[4];            // regions E0, RA, RB, E1 (leader CTA's copies are the ones used)
   SchedRing sched;
+  uint64_t cancel_bar;              // drawing thread: completion of its try_cancel
+  alignas(16) uint4 cancel_response;
   uint32_t tmem_base;
   int abort_flag;
 };
 
-enum { GM_IN = 0, GM_OUT = 1, GM_IN_SMALL = 2 };  // per-expert tensor-map slots of the forward / dX kernels
+enum { GM_IN = 0, GM_OUT = 1 };  // per-expert tensor-map slots (GM_IN: NF4 kernel only; GM_OUT: also scattered outputs)
 enum { REG_E0 = 0, REG_RA = 1, REG_RB = 2, REG_E1 = 3 };
 constexpr int PAIR_STAGING_BYTES = 32 * 128;  // 32 tokens x 64 weight rows x 16 bit
 
 enum PairWaitCode { PW_EMPTY = 11, PW_FULL = 12, PW_TMEM_EMPTY = 13, PW_TMEM_FULL = 14, PW_PEER = 15,
-                    PW_SCHED_FULL = 17, PW_SCHED_EMPTY = 18, PW_SCHED_VALUE = 19 };
+                    PW_SCHED_FULL = 17, PW_SCHED_EMPTY = 18, PW_SCHED_VALUE = 19, PW_CANCEL = 20 };
 
 template <typename T>
 __device__ __forceinline__ void store_scalar(void* out, int64_t idx, float v) {
   reinterpret_cast<T*>(out)[idx] = from_f32<T>(v);
 }
 
+// Rows [t0, t_end) (fewer than 32) of a staged round, CHUNKS x 16 bytes each, to the output from column n0 on.
+// Columns end at N, a multiple of 8, so a chunk is stored whole or not at all.
+template <int CHUNKS>
+__device__ __forceinline__ void store_clipped_rows(const uint8_t* buf, uint8_t* out, int t0, int t_end, int n0, int N, int epi_tid) {
+  for (int i = epi_tid; i < (t_end - t0) * CHUNKS; i += 128) {
+    const int r = i / CHUNKS, q = i % CHUNKS;
+    const int n = n0 + q * 8;
+    if (n < N)
+      *reinterpret_cast<uint4*>(out + ((int64_t)(t0 + r) * N + n) * 2) =
+          *reinterpret_cast<const uint4*>(buf + (q >> 3) * PAIR_STAGING_BYTES + r * 128 + (((q & 7) ^ (r & 7)) << 4));
+  }
+}
+
 // Epilogue of one accumulator (n_mma token columns of this CTA's 128 weight rows) for 16-bit
 // outputs: TMEM is read in the accumulator-fragment shape, packed to 16 bit and transposed by
 // stmatrix into a swizzled [token][weight row] staging tile (32 tokens x 2 x 64 weight rows per
-// round, double buffered), which leaves through TMA stores; `my` is the expert's output map,
-// so rows past the group's end and columns past N are clipped.  Called by the 128 epilogue
-// threads (warps 2..5); `staging` holds 4 * PAIR_STAGING_BYTES.
+// round, double buffered), which leaves through TMA stores; columns past N are clipped by the map `my`.
+// Rows: with `out` == nullptr `my` is the group's own map and clips them too; otherwise `my` covers the whole
+// output and a round that reaches past `t_end` is copied from the staging tile instead.
+// Called by the 128 epilogue threads (warps 2..5); `staging` holds 4 * PAIR_STAGING_BYTES.
 __device__ __forceinline__ void pair_store_tile_staged(uint8_t* staging, uint32_t& chunk_it, uint32_t taddr, int n_mma,
                                                        int quarter, int lane, int epi_tid, bool is_bf16,
-                                                       const CUtensorMap* my, int n_cta, int t0, int N) {
+                                                       const CUtensorMap* my, int n_cta, int t0, int N,
+                                                       uint8_t* out = nullptr, int t_end = 0) {
   const int half = quarter >> 1;
   const int chunk = 4 * (quarter & 1) + (lane >> 3);  // 16-byte chunk of the 128-byte staging row
 #pragma unroll 1
@@ -128,10 +165,14 @@ __device__ __forceinline__ void pair_store_tile_staged(uint8_t* staging, uint32_
     }
     fence_proxy_async_smem();
     named_barrier_sync(1, 128);
+    const bool clip = out != nullptr && t_end - (t0 + c) < 32;
+    if (clip) store_clipped_rows<16>(buf, out, t0 + c, t_end, n_cta, N, epi_tid);
     if (epi_tid == 0) {
-      tma_store_2d(my, buf, n_cta, t0 + c);
-      if (n_cta + 64 < N) tma_store_2d(my, buf + PAIR_STAGING_BYTES, n_cta + 64, t0 + c);
-      tma_store_commit();
+      if (!clip) {
+        tma_store_2d(my, buf, n_cta, t0 + c);
+        if (n_cta + 64 < N) tma_store_2d(my, buf + PAIR_STAGING_BYTES, n_cta + 64, t0 + c);
+      }
+      tma_store_commit();  // (an empty group keeps the count of the wait above)
     }
   }
 }
@@ -154,7 +195,8 @@ __device__ __forceinline__ float gate_up_one(float acc_gate, float acc_up) {
 // 8 tokens); the CTA's four warps fill a [32 tokens][64 features] tile that leaves by TMA.
 __device__ __forceinline__ void pair_store_tile_gate_up(uint8_t* staging, uint32_t& chunk_it, uint32_t taddr, int n_mma,
                                                         int quarter, int lane, int epi_tid, bool is_bf16,
-                                                        const CUtensorMap* my, int feat_cta, int t0, int n_feat) {
+                                                        const CUtensorMap* my, int feat_cta, int t0, int n_feat,
+                                                        uint8_t* out, int t_end) {
   const int chunk = 2 * quarter + ((lane >> 3) & 1);  // 16-byte chunk of the 128-byte staging row
 #pragma unroll 1
   for (int c = 0; c < n_mma; c += 32, ++chunk_it) {
@@ -180,8 +222,10 @@ __device__ __forceinline__ void pair_store_tile_gate_up(uint8_t* staging, uint32
     }
     fence_proxy_async_smem();
     named_barrier_sync(1, 128);
+    const bool clip = t_end - (t0 + c) < 32;
+    if (clip) store_clipped_rows<8>(buf, out, t0 + c, t_end, feat_cta, n_feat, epi_tid);
     if (epi_tid == 0) {
-      if (feat_cta < n_feat) tma_store_2d(my, buf, feat_cta, t0 + c);  // columns past the last feature are clipped
+      if (!clip && feat_cta < n_feat) tma_store_2d(my, buf, feat_cta, t0 + c);  // columns past the last feature are clipped
       tma_store_commit();
     }
   }
@@ -245,6 +289,22 @@ struct TileFeed {
       if (!publish(tile) || tile < 0) return;
     }
   }
+  // The same with the tiles of the clusters that have not started yet: `first` is this cluster's own tile;
+  // ids from `total` on (the grid is an upper bound) are passed over.
+  __device__ __forceinline__ void run_cancel(uint64_t* bar, uint4* response, int total, int first) {
+    uint32_t ph = 0;
+    for (int tile = first;;) {
+      if (tile < total && !publish(tile)) return;
+      mbar_expect_tx(bar, 16);
+      cluster_try_cancel(response, bar);
+      if (!mbar_wait(bar, ph, abort_flag, PW_CANCEL)) return;
+      ph ^= 1;
+      const int cta = cluster_cancelled_cta(response);
+      fence_proxy_async_smem();  // the response has been read before the next one may be written
+      if (cta < 0) { publish(-1); return; }
+      tile = cta >> 1;
+    }
+  }
   // a reader (one thread): next tile id, or -1 when there are no more (or the wait was abandoned)
   __device__ __forceinline__ int take() {
     const uint32_t q = n % SCHED_DEPTH, ph = (n / SCHED_DEPTH) & 1;
@@ -300,11 +360,13 @@ __device__ __forceinline__ uint32_t pair_regions(uint32_t parity, int n_main, in
 // [gate f..f+15][up f..f+15]... so that a warp's quarter of TMEM holds gate and up of the same 16
 // features; the epilogue writes h = silu(gate) * up (p.N = I columns) and neither projection.
 // ---------------------------------------------------------------------------------------
-template <bool W_MN, bool GATE_UP = false, bool GATHER = false>
+//
+// MULTI: maps.n_seg operand pairs (the other forms have one), each with its own contraction length.
+template <bool W_MN, bool GATE_UP = false, bool GATHER = false, bool MULTI = false>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1)
-pair_fwd_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x,
-                const GemmParams p, const __grid_constant__ CUtensorMap tmap_w2) {
+pair_fwd_kernel(const __grid_constant__ PairMaps maps, const GemmParams p) {
   static_assert(!(W_MN && GATE_UP), "the fused gate/up form reads K-major weights");
+  static_assert(!(MULTI && (GATE_UP || GATHER)), "several operand pairs: plain forward and dX only");
   static_assert(!(W_MN && GATHER), "rows are gathered in the forward forms only");
   constexpr int TILE_N = GATE_UP ? 128 : 256;  // output columns (features) per pair
   constexpr int STAGE_BYTES = PAIR_STAGE_BYTES;
@@ -323,35 +385,30 @@ pair_fwd_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constan
   const int lane = threadIdx.x & 31;
   const uint32_t rank = cluster_ctarank();
   const bool leader = rank == 0;
-  // tails and small boxes need the per-expert small-box maps
-  const bool small_maps = p.group_maps != nullptr && p.small_maps;
-  const int tail = (small_maps || GATHER) ? PAIR_TAIL : 0;
-
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) { mbar_init(&ctl->full[s], 1); mbar_init(&ctl->empty[s], 1); }
     for (int a = 0; a < 2; ++a) mbar_init(&ctl->tmem_full[a], 1);
     for (int r = 0; r < 4; ++r) mbar_init(&ctl->tmem_free[r], 8);
     TileFeed<2>::init(&ctl->sched);
+    mbar_init(&ctl->cancel_bar, 1);
     ctl->abort_flag = 0;
     fence_barrier_init();
-    tma_prefetch_desc(&tmap_w);
-    tma_prefetch_desc(&tmap_x);
+    tma_prefetch_desc(&maps.w[0]);
+    tma_prefetch_desc(&maps.x[0]);
   }
   if (warp == 1) {
     tmem_alloc_pair(&ctl->tmem_base, TMEM_COLS);
     tmem_relinquish_pair();
   }
-  build_group_tables(p.m_sizes, p.ms64, p.E, p.M, PAIR_TOKENS, row_start, tt_start, tail);
+  build_group_tables(p.m_sizes, p.ms64, p.E, p.M, PAIR_TOKENS, row_start, tt_start, PAIR_TAIL);
   tc_fence_before_sync();
   cluster_sync_all();  // barriers of both CTAs are initialised before anybody signals them
   tc_fence_after_sync();
   const uint32_t tmem_base = ctl->tmem_base;
 
   const int n_tiles = (p.N + TILE_N - 1) / TILE_N;  // 256 weight rows per pair
-  const int k_blocks = (p.K + BK - 1) / BK;
+  const int n_seg = MULTI ? maps.n_seg : 1;
   const int64_t total_tiles = (int64_t)tt_start[p.E] * n_tiles;
-  const int pair_id = blockIdx.x >> 1;
-  const int num_pairs = gridDim.x >> 1;
 
   // tile index -> tile.  Within an expert the token tile varies fastest, so neighbouring tiles
   // (which run at about the same time) read the same weight slice.
@@ -368,7 +425,7 @@ pair_fwd_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constan
     const int left = t.t_end - t.t0;
     if (left >= PAIR_TOKENS) {
       t.n_main = PAIR_TOKENS;
-      t.n_tail = (jt == tt_e - 1) ? ((left - PAIR_TOKENS + 15) & ~15) : 0;  // at most `tail` by the tile count
+      t.n_tail = (jt == tt_e - 1) ? ((left - PAIR_TOKENS + 15) & ~15) : 0;  // at most PAIR_TAIL by the tile count
     } else {
       t.n_main = (left + 15) & ~15;
       t.n_tail = 0;
@@ -379,7 +436,7 @@ pair_fwd_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constan
   // PAIR_SMALL_BOX rows, and bytes both CTAs' loads of the stage bring in
   auto main_small_boxes = [&](int n_main) {  // 0: one 128-row box
     const int rows = n_main >> 1;
-    return (small_maps && rows <= 64) ? (rows + PAIR_SMALL_BOX - 1) / PAIR_SMALL_BOX : 0;
+    return rows <= 64 ? (rows + PAIR_SMALL_BOX - 1) / PAIR_SMALL_BOX : 0;
   };
   auto tail_boxes = [&](int n_tail) { return ((n_tail >> 1) + PAIR_SMALL_BOX - 1) / PAIR_SMALL_BOX; };
 
@@ -412,7 +469,7 @@ pair_fwd_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constan
       }
       const bool has_main = 4 * lane < rows_main, has_tail = 4 * lane < rows_tail;
       const uint32_t b_bytes = (uint32_t)(rows_main + rows_tail) * (BK * 2);
-      for (int kb = 0; kb < k_blocks; ++kb) {
+      for (int kb = 0; kb < maps.kb[0]; ++kb) {
         uint8_t* sa = smem + s * STAGE_BYTES;
         uint8_t* sb = sa + PAIR_HALF_BYTES;
         const uint32_t bar = full_leader0 + s * 8;
@@ -425,18 +482,18 @@ pair_fwd_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constan
               const int feat = t.n0 + (int)rank * 64;
 #pragma unroll
               for (int q = 0; q < 4; ++q) {
-                tma_load_3d_pair(sa + (2 * q) * 2048, &tmap_w, bar, kb * BK, feat + 16 * q, we);
-                tma_load_3d_pair(sa + (2 * q + 1) * 2048, &tmap_w2, bar, kb * BK, feat + 16 * q, we);
+                tma_load_3d_pair(sa + (2 * q) * 2048, &maps.w[0], bar, kb * BK, feat + 16 * q, we);
+                tma_load_3d_pair(sa + (2 * q + 1) * 2048, &maps.w[1], bar, kb * BK, feat + 16 * q, we);
               }
             } else {
-              tma_load_3d_pair(sa, &tmap_w, bar, kb * BK, w_row, we);
+              tma_load_3d_pair(sa, &maps.w[0], bar, kb * BK, w_row, we);
             }
           }
         }
         go = __shfl_sync(0xffffffffu, go, 0);  // the stage is free (and its byte count announced) for every lane
         if (!go) { ok = false; break; }
-        if (has_main) tma_gather4_pair(sb + lane * (4 * BK * 2), &tmap_x, bar, kb * BK, mr[0], mr[1], mr[2], mr[3]);
-        if (has_tail) tma_gather4_pair(sb + PAIR_HALF_BYTES + lane * (4 * BK * 2), &tmap_x, bar, kb * BK, tr[0], tr[1], tr[2], tr[3]);
+        if (has_main) tma_gather4_pair(sb + lane * (4 * BK * 2), &maps.x[0], bar, kb * BK, mr[0], mr[1], mr[2], mr[3]);
+        if (has_tail) tma_gather4_pair(sb + PAIR_HALF_BYTES + lane * (4 * BK * 2), &maps.x[0], bar, kb * BK, tr[0], tr[1], tr[2], tr[3]);
         if (++s == STAGES) { s = 0; ph ^= 1; }
       }
     }
@@ -445,11 +502,9 @@ pair_fwd_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constan
     if (elect_one()) {
       TileFeed<2> feed(&ctl->sched, abort_flag);
       const uint32_t full_leader0 = map_to_cta(smem_u32(&ctl->full[0]), 0);
-      uint32_t it = 0;
       int s = 0;
       uint32_t ph = 0;
       bool ok = true;
-      int last_e = -1;
       while (ok) {
         const int tile = feed.take();
         if (tile < 0) break;
@@ -458,45 +513,42 @@ pair_fwd_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constan
         const int w_row = t.n0 + (int)rank * 128;
         const int tok = t.t0 + (int)rank * (t.n_main >> 1);
         const int tok_tail = t.t0 + PAIR_TOKENS + (int)rank * (t.n_tail >> 1);
-        // with per-expert maps the token rows past the group's end are zero-filled, not fetched
-        const CUtensorMap* mx = p.group_maps ? p.group_maps + (size_t)GM_IN * p.E + t.e : &tmap_x;
-        const CUtensorMap* ms = small_maps ? p.group_maps + (size_t)GM_IN_SMALL * p.E + t.e : nullptr;
-        if (p.group_maps && t.e != last_e) {
-          tensormap_acquire(mx);
-          if (ms) tensormap_acquire(ms);
-          last_e = t.e;
-        }
         const int nsb = main_small_boxes(t.n_main);
         const int ntb = tail_boxes(t.n_tail);
         const uint32_t b_bytes = (nsb ? nsb * PAIR_SMALL_BOX * BK * 2 : PAIR_HALF_BYTES) + ntb * PAIR_SMALL_BOX * BK * 2;
-        for (int kb = 0; kb < k_blocks; ++kb, ++it) {
-          if (!mbar_wait(&ctl->empty[s], ph ^ 1, abort_flag, PW_EMPTY)) { ok = false; break; }
-          uint8_t* sa = smem + s * STAGE_BYTES;
-          uint8_t* sb = sa + PAIR_HALF_BYTES;
-          const uint32_t bar = full_leader0 + s * 8;
-          if (leader) mbar_expect_tx(&ctl->full[s], 2 * (PAIR_HALF_BYTES + b_bytes));  // both CTAs' bytes
-          if constexpr (GATE_UP) {
-            const int feat = t.n0 + (int)rank * 64;  // this CTA's 64 features
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-              tma_load_3d_pair(sa + (2 * q) * 2048, &tmap_w, bar, kb * BK, feat + 16 * q, we);
-              tma_load_3d_pair(sa + (2 * q + 1) * 2048, &tmap_w2, bar, kb * BK, feat + 16 * q, we);
+        for (int i = 0; i < n_seg && ok; ++i) {
+          const CUtensorMap* mw = &maps.w[i];
+          const CUtensorMap* mx = &maps.x[i];
+          const CUtensorMap* ms = &maps.xs[i];
+          for (int kb = 0; kb < maps.kb[i]; ++kb) {
+            if (!mbar_wait(&ctl->empty[s], ph ^ 1, abort_flag, PW_EMPTY)) { ok = false; break; }
+            uint8_t* sa = smem + s * STAGE_BYTES;
+            uint8_t* sb = sa + PAIR_HALF_BYTES;
+            const uint32_t bar = full_leader0 + s * 8;
+            if (leader) mbar_expect_tx(&ctl->full[s], 2 * (PAIR_HALF_BYTES + b_bytes));  // both CTAs' bytes
+            if constexpr (GATE_UP) {
+              const int feat = t.n0 + (int)rank * 64;  // this CTA's 64 features
+  #pragma unroll
+              for (int q = 0; q < 4; ++q) {
+                tma_load_3d_pair(sa + (2 * q) * 2048, mw, bar, kb * BK, feat + 16 * q, we);
+                tma_load_3d_pair(sa + (2 * q + 1) * 2048, &maps.w[1], bar, kb * BK, feat + 16 * q, we);
+              }
+            } else if constexpr (!W_MN) {
+              tma_load_3d_pair(sa, mw, bar, kb * BK, w_row, we);
+            } else {
+              tma_load_3d_pair(sa, mw, bar, w_row, kb * BK, we);
+              tma_load_3d_pair(sa + BK * 128, mw, bar, w_row + 64, kb * BK, we);
             }
-          } else if constexpr (!W_MN) {
-            tma_load_3d_pair(sa, &tmap_w, bar, kb * BK, w_row, we);
-          } else {
-            tma_load_3d_pair(sa, &tmap_w, bar, w_row, kb * BK, we);
-            tma_load_3d_pair(sa + BK * 128, &tmap_w, bar, w_row + 64, kb * BK, we);
+            if (nsb == 0) {
+              tma_load_2d_pair(sb, mx, bar, kb * BK, tok);
+            } else {
+              for (int b = 0; b < nsb; ++b)
+                tma_load_2d_pair(sb + b * (PAIR_SMALL_BOX * BK * 2), ms, bar, kb * BK, tok + b * PAIR_SMALL_BOX);
+            }
+            for (int b = 0; b < ntb; ++b)
+              tma_load_2d_pair(sb + PAIR_HALF_BYTES + b * (PAIR_SMALL_BOX * BK * 2), ms, bar, kb * BK, tok_tail + b * PAIR_SMALL_BOX);
+            if (++s == STAGES) { s = 0; ph ^= 1; }
           }
-          if (nsb == 0) {
-            tma_load_2d_pair(sb, mx, bar, kb * BK, tok);
-          } else {
-            for (int b = 0; b < nsb; ++b)
-              tma_load_2d_pair(sb + b * (PAIR_SMALL_BOX * BK * 2), ms, bar, kb * BK, tok + b * PAIR_SMALL_BOX);
-          }
-          for (int b = 0; b < ntb; ++b)
-            tma_load_2d_pair(sb + PAIR_HALF_BYTES + b * (PAIR_SMALL_BOX * BK * 2), ms, bar, kb * BK, tok_tail + b * PAIR_SMALL_BOX);
-          if (++s == STAGES) { s = 0; ph ^= 1; }
         }
       }
     }
@@ -505,7 +557,7 @@ pair_fwd_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constan
     if (!leader) {
       if (elect_one()) {
         TileFeed<2> feed(&ctl->sched, abort_flag);
-        feed.run(p.tile_counter, (int)total_tiles, pair_id, num_pairs);
+        feed.run_cancel(&ctl->cancel_bar, &ctl->cancel_response, (int)total_tiles, (int)(blockIdx.x >> 1));
       }
     } else if (elect_one()) {
       TileFeed<2> feed(&ctl->sched, abort_flag);
@@ -533,33 +585,45 @@ pair_fwd_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constan
         tc_fence_after_sync();
         const uint32_t d_main = tmem_base + (par ? PAIR_TOKENS : 0);
         const uint32_t d_tail = tmem_base + (par ? PAIR_TOKENS - PAIR_TAIL : PAIR_TOKENS);
-        // Two copies of the k-loop, with and without the tail MMAs: a test of n_tail between the
-        // MMAs of one loop costs the issuing thread a quarter of its rate.
-        auto k_loop = [&](auto has_tail) {
-          for (int kb = 0; kb < k_blocks; ++kb) {
-            if (!mbar_wait_cluster(&ctl->full[s], ph, abort_flag, PW_FULL)) { ok = false; break; }
-            tc_fence_after_sync();
-            const uint32_t sa = smem_u32(smem + s * STAGE_BYTES);
-            const uint32_t sb = sa + PAIR_HALF_BYTES;
-            const uint64_t da = W_MN ? make_smem_desc(sa, BK * 128, 1024) : make_smem_desc(sa, 16, 1024);
-            const uint64_t db = make_smem_desc(sb, 16, 1024);
+        // One block of 64 of the contraction.  Compiled with and without the tail MMAs, and with all steps or a
+        // counted number of them: a test between the MMAs of one block costs the issuing thread a quarter of its rate.
+        auto block = [&](auto has_tail, auto all_steps, int steps, bool first) {
+          if (!mbar_wait_cluster(&ctl->full[s], ph, abort_flag, PW_FULL)) { ok = false; return; }
+          tc_fence_after_sync();
+          const uint32_t sa = smem_u32(smem + s * STAGE_BYTES);
+          const uint32_t sb = sa + PAIR_HALF_BYTES;
+          const uint64_t da = W_MN ? make_smem_desc(sa, BK * 128, 1024) : make_smem_desc(sa, 16, 1024);
+          const uint64_t db = make_smem_desc(sb, 16, 1024);
+          const uint64_t dbt = make_smem_desc(sb + PAIR_HALF_BYTES, 16, 1024);
+          auto step = [&](int k, uint32_t d, uint64_t desc_b, uint32_t idesc) {
+            const uint64_t b_adv = (uint64_t)((k * UMMA_K * 2) >> 4);
+            const uint64_t a_adv = W_MN ? (uint64_t)((k * UMMA_K * 128) >> 4) : b_adv;
+            umma_f16_pair(d, da + a_adv, desc_b + b_adv, idesc, !first || k != 0);
+          };
+          if constexpr (decltype(all_steps)::value) {
 #pragma unroll
-            for (int k = 0; k < BK / UMMA_K; ++k) {
-              const uint64_t b_adv = (uint64_t)((k * UMMA_K * 2) >> 4);
-              const uint64_t a_adv = W_MN ? (uint64_t)((k * UMMA_K * 128) >> 4) : b_adv;
-              umma_f16_pair(d_main, da + a_adv, db + b_adv, idesc_main, (kb | k) != 0);
-            }
+            for (int k = 0; k < BK / UMMA_K; ++k) step(k, d_main, db, idesc_main);
             if constexpr (decltype(has_tail)::value) {
-              const uint64_t dbt = make_smem_desc(sb + PAIR_HALF_BYTES, 16, 1024);
 #pragma unroll
-              for (int k = 0; k < BK / UMMA_K; ++k) {
-                const uint64_t b_adv = (uint64_t)((k * UMMA_K * 2) >> 4);
-                const uint64_t a_adv = W_MN ? (uint64_t)((k * UMMA_K * 128) >> 4) : b_adv;
-                umma_f16_pair(d_tail, da + a_adv, dbt + b_adv, idesc_tail, (kb | k) != 0);
-              }
+              for (int k = 0; k < BK / UMMA_K; ++k) step(k, d_tail, dbt, idesc_tail);
             }
-            umma_commit_pair(&ctl->empty[s], 3);
-            if (++s == STAGES) { s = 0; ph ^= 1; }
+          } else {
+#pragma unroll 1
+            for (int k = 0; k < steps; ++k) {
+              step(k, d_main, db, idesc_main);
+              if constexpr (decltype(has_tail)::value) step(k, d_tail, dbt, idesc_tail);
+            }
+          }
+          umma_commit_pair(&ctl->empty[s], 3);
+          if (++s == STAGES) { s = 0; ph ^= 1; }
+        };
+        auto k_loop = [&](auto has_tail) {
+          for (int i = 0; i < n_seg && ok; ++i) {
+            // (one operand pair: rows past the contraction's end are zeros in both operands and cost nothing to add)
+            const bool partial = MULTI && maps.last_steps[i] < BK / UMMA_K;
+            const int full_blocks = maps.kb[i] - (partial ? 1 : 0);
+            for (int kb = 0; kb < full_blocks && ok; ++kb) block(has_tail, std::true_type{}, BK / UMMA_K, (i | kb) == 0);
+            if (MULTI && partial && ok) block(has_tail, std::false_type{}, maps.last_steps[i], (i | full_blocks) == 0);
           }
         };
         if (t.n_tail) k_loop(std::true_type{}); else k_loop(std::false_type{});
@@ -573,8 +637,10 @@ pair_fwd_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constan
     const int quarter = warp & 3;
     const int epi_tid = threadIdx.x - 64;  // 0..127
     const uint32_t tmem_free_leader0 = map_to_cta(smem_u32(&ctl->tmem_free[0]), 0);
-    // 16-bit outputs with per-expert output maps leave through shared memory and TMA stores
-    const bool staged = p.group_maps != nullptr && p.dtype_out != MOE_F32;
+    // 16-byte aligned 16-bit outputs leave through shared memory and TMA stores; group_maps: scattered outputs,
+    // one map per group that re-bases and clips it
+    const bool staged = p.staged;
+    uint8_t* const clip_out = p.group_maps != nullptr ? nullptr : reinterpret_cast<uint8_t*>(p.out);
     const bool is_bf16 = p.dtype_out == MOE_BF16;
     uint32_t seq = 0, chunk_it = 0;
     int last_e = -1;
@@ -586,8 +652,8 @@ pair_fwd_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constan
       const uint32_t full_ph = (seq >> 1) & 1;
       const int n = t.n0 + (int)rank * 128 + quarter * 32 + lane;  // this thread's weight row = output column
       const bool n_ok = n < p.N;
-      const CUtensorMap* my = staged ? p.group_maps + (size_t)GM_OUT * p.E + t.e : nullptr;
-      if (staged && epi_tid == 0 && t.e != last_e) { tensormap_acquire(my); last_e = t.e; }
+      const CUtensorMap* my = p.group_maps != nullptr ? p.group_maps + (size_t)GM_OUT * p.E + t.e : &maps.out;
+      if (p.group_maps != nullptr && epi_tid == 0 && t.e != last_e) { tensormap_acquire(my); last_e = t.e; }
       if (named_barrier_any(2, 128, !mbar_wait_cluster(&ctl->tmem_full[par], full_ph, abort_flag, PW_TMEM_FULL))) break;
       tc_fence_after_sync();
       const uint32_t lane_base = tmem_base + ((uint32_t)(quarter * 32) << 16);
@@ -596,12 +662,12 @@ pair_fwd_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constan
       auto drain = [&](int col, int n_cols, int tok0) {
         const uint32_t taddr = lane_base + (uint32_t)col;
         if constexpr (GATE_UP) {
-          // (the host only launches this form with per-expert output maps and a 16-bit output)
+          // (the host only launches this form with a staged 16-bit output)
           pair_store_tile_gate_up(staging, chunk_it, taddr, n_cols, quarter, lane, epi_tid, is_bf16, my,
-                                  t.n0 + (int)rank * 64, tok0, p.N);
+                                  t.n0 + (int)rank * 64, tok0, p.N, reinterpret_cast<uint8_t*>(p.out), t.t_end);
         } else if (staged) {
           pair_store_tile_staged(staging, chunk_it, taddr, n_cols, quarter, lane, epi_tid, is_bf16, my,
-                                 t.n0 + (int)rank * 128, tok0, p.N);
+                                 t.n0 + (int)rank * 128, tok0, p.N, clip_out, t.t_end);
         } else {
 #pragma unroll 1
           for (int c = 0; c < n_cols; c += 32) {
