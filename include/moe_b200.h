@@ -104,11 +104,11 @@ int moe_batch_begins_ends(const void* s_sorted, int s_dtype, int64_t M, int E,
  * consecutive rows (m_sizes_dtype MOE_I32 or MOE_I64, sum = M, zeros allowed).
  * Accumulation is fp32; the result is rounded once to dtype_out.
  * ws/ws_bytes: device scratch of moe_grouped_gemm_workspace_bytes() bytes, 128-byte aligned,
- *   owned by the caller.  A small launch ahead of each GEMM writes per-expert tensor maps and a
- *   work-item counter into it, so one workspace serves one GEMM at a time: calls issued on one
- *   stream may share it, calls on different streams need one each.  Forward and dX also accept
- *   NULL/0 and then run a slower form (no per-expert maps, fixed tile order); dW on the
- *   tensor-core path and the fused / gathered / scattered forms return MOE_ERR_WORKSPACE.
+ *   owned by the caller.  dW, the NF4 and the scattered forms launch a small kernel ahead of the
+ *   GEMM that writes per-expert tensor maps and a work-item counter into it, so one workspace serves
+ *   one GEMM at a time: calls issued on one stream may share it, calls on different streams need one
+ *   each.  Forward and dX accept NULL/0 (they do not use it); dW on the tensor-core path and the
+ *   fused / gathered / scattered forms return MOE_ERR_WORKSPACE.
  * ------------------------------------------------------------------------------- */
 size_t moe_grouped_gemm_workspace_bytes(int which /*0 fwd, 1 dx, 2 dw*/, int64_t M, int N, int K, int E);
 
@@ -250,6 +250,27 @@ int moe_combine(const void* y, const int32_t* inv_sort_idx, const void* weights,
  * Replaces the autograd of qwen3_moe_fused/modular_qwen3_moe_fused.py:110-115. */
 int moe_combine_bwd(const void* dout, const void* y, const int32_t* inv_sort_idx, const void* weights, void* dy,
                     void* dweights, int64_t T, int k, int H, int dtype, void* stream);
+
+/* y = sum_i x_i W_i^T (which = 0, W_i (E, N, K_i)) or sum_i x_i W_i (which = 1, W_i (E, K_i, N)) per expert, the n <= 4
+ * operand pairs contracted into one fp32 accumulator and rounded once.  x_i has M rows of K_i elements, ldx[i] apart.
+ * Host arrays x, ldx, w, K of n entries.  16-bit dtypes, N >= 192, extents and pitches multiples of 8, 16-byte aligned
+ * bases; MOE_ERR_UNSUPPORTED otherwise, or when another kernel family is selected.  No workspace.
+ * Replaces the base product + LoRA product sums of qwen3_moe_fused/kernels/fast_lora.py:101-110,128-153. */
+int moe_grouped_gemm_sum(int which, int n, const void* const* x, const int64_t* ldx, const void* const* w, const int* K,
+                         const void* m_sizes, int msd, void* y, int64_t M, int N, int E, int dtype, void* stream);
+
+/* Thin projections with a factor applied to the fp32 accumulator.  which = 0: y[:, 0:n0] = s0 * x a0^T and, if a1 is
+ * given, y[:, n0:n0+n1] = s1 * x a1^T with a_i (E, n_i, K), x read once; which = 1: y[:, 0:n0] = s0 * x a0 with a0
+ * (E, K, n0).  Rows of y are ldy elements apart.  16-bit dtypes, n0 + n1 <= 256, extents and ldy multiples of 8,
+ * 16-byte aligned bases; MOE_ERR_UNSUPPORTED otherwise.
+ * Replaces the first factor of each LoRA product, qwen3_moe_fused/kernels/fast_lora.py:101-110. */
+int moe_lora_project(int which, const void* x, const void* a0, int n0, float s0, const void* a1, int n1, float s1,
+                     const void* m_sizes, int msd, void* y, int64_t ldy, int64_t M, int K, int E, int dtype, void* stream);
+
+/* moe_grouped_gemm_dw on operands whose rows are ldx / ldy elements apart (multiples of 8; dtype in = dtype out).
+ * Replaces qwen3_moe_fused/kernels/fast_lora.py:139-149 together with moe_lora_project. */
+int moe_grouped_gemm_dw_strided(const void* x, int64_t ldx, const void* dy, int64_t ldy, const void* m_sizes, int msd,
+                                void* w, int64_t M, int N, int K, int E, int dtype, void* ws, size_t ws_bytes, void* stream);
 
 /* ---------------------------------------------------------------------------------
  * Expert parallelism over peer memory.  The reference has no multi-GPU path

@@ -30,6 +30,14 @@ int tc_gate_up_silu(const void* x, const void* w_gate, const void* w_up, const v
 int tc_grouped_gemm_gather(const void* x, int64_t x_rows, const int* row_index, int index_div, const void* w,
                            const void* m_sizes, int ms64, void* y, int64_t M, int N, int K, int E, int dtype_in,
                            int dtype_out, void* ws, size_t ws_bytes, cudaStream_t stream);
+int tc_grouped_gemm_sum(int which, int n, const void* const* x, const int64_t* ldx, const void* const* w, const int* K,
+                        const void* m_sizes, int ms64, void* out, int64_t M, int N, int E, int dtype, cudaStream_t stream);
+int tc_lora_project(int which, const void* x, const void* a0, int n0, float s0, const void* a1, int n1, float s1,
+                    const void* m_sizes, int ms64, void* out, int ld_out, int64_t M, int K, int E, int dtype,
+                    cudaStream_t stream);
+int tc_grouped_gemm_dw_strided(const void* x, int64_t ldx, const void* dy, int64_t ldy, const void* m_sizes, int ms64,
+                               void* out, int64_t M, int N, int K, int E, int dtype, void* ws, size_t ws_bytes,
+                               cudaStream_t stream);
 int tc_read_error(int* flag_out, bool clear);
 size_t tc_workspace_bytes(int E);
 int tc_read_late_values(int* out);
@@ -217,6 +225,61 @@ MOE_API int moe_grouped_gemm_fwd_gather(const void* x, int64_t x_rows, const int
   if (K == 0 || x_rows == 0 || !tc_eligible(0, x, w, y, M, N, K, E, dtype_in, dtype_out)) return MOE_ERR_UNSUPPORTED;
   return tc_grouped_gemm_gather(x, x_rows, row_index, index_div, w, m_sizes, msd == MOE_I64, y, M, N, K, E, dtype_in,
                                 dtype_out, ws, ws_bytes, (cudaStream_t)stream);
+}
+
+// Contractions of several (activation, weight) pairs summed in one accumulator.  Tensor-core CTA-pair kernel only.
+MOE_API int moe_grouped_gemm_sum(int which, int n, const void* const* x, const int64_t* ldx, const void* const* w,
+                                 const int* K, const void* m_sizes, int msd, void* y, int64_t M, int N, int E, int dtype,
+                                 void* stream) {
+  if ((which != 0 && which != 1) || n < 1 || n > 4) return MOE_ERR_SHAPE;
+  if (!x || !ldx || !w || !K) return MOE_ERR_NULL;
+  for (int i = 0; i < n; ++i) {
+    const int st = check_common(x[i], w[i], m_sizes, msd, y, M, N, K[i], E, dtype, dtype);
+    if (st != MOE_OK) return st;
+    if (ldx[i] < K[i]) return MOE_ERR_SHAPE;
+  }
+  if (M == 0 || N == 0) return MOE_OK;
+  if (!device_is_sm100()) return MOE_ERR_DEVICE;
+  const int path = g_path.load(std::memory_order_relaxed);
+  if (path == MOE_PATH_SIMT || path == MOE_PATH_TC_SINGLE || N < 192 || ((uintptr_t)y & 15)) return MOE_ERR_UNSUPPORTED;
+  for (int i = 0; i < n; ++i)
+    if (ldx[i] % 8 || !tc_eligible(which, x[i], w[i], y, M, N, K[i], E, dtype, dtype)) return MOE_ERR_UNSUPPORTED;
+  return tc_grouped_gemm_sum(which, n, x, ldx, w, K, m_sizes, msd == MOE_I64, y, M, N, E, dtype, (cudaStream_t)stream);
+}
+
+MOE_API int moe_lora_project(int which, const void* x, const void* a0, int n0, float s0, const void* a1, int n1, float s1,
+                             const void* m_sizes, int msd, void* y, int64_t ldy, int64_t M, int K, int E, int dtype,
+                             void* stream) {
+  if (which != 0 && which != 1) return MOE_ERR_SHAPE;
+  int st = check_common(x, a0, m_sizes, msd, y, M, n0, K, E, dtype, dtype);
+  if (st != MOE_OK) return st;
+  if (a1 && (which != 0 || n1 <= 0)) return MOE_ERR_SHAPE;
+  const int n = n0 + (a1 ? n1 : 0);
+  if (ldy < n || ldy > 0x7fffffffLL) return MOE_ERR_SHAPE;
+  if (M == 0 || n0 == 0) return MOE_OK;
+  if (!device_is_sm100()) return MOE_ERR_DEVICE;
+  const int path = g_path.load(std::memory_order_relaxed);
+  if (path == MOE_PATH_SIMT || n > 256 || n0 % 8 || n % 8 || ldy % 8 || ((uintptr_t)y & 15) || ((uintptr_t)a1 & 15) ||
+      !tc_eligible(which, x, a0, y, M, n, K, E, dtype, dtype))
+    return MOE_ERR_UNSUPPORTED;
+  return tc_lora_project(which, x, a0, n0, s0, a1, n1, s1, m_sizes, msd == MOE_I64, y, (int)ldy, M, K, E, dtype,
+                         (cudaStream_t)stream);
+}
+
+MOE_API int moe_grouped_gemm_dw_strided(const void* x, int64_t ldx, const void* dy, int64_t ldy, const void* m_sizes,
+                                        int msd, void* w, int64_t M, int N, int K, int E, int dtype, void* ws,
+                                        size_t ws_bytes, void* stream) {
+  if (!is_float_dtype(dtype) || !is_int_dtype(msd)) return MOE_ERR_DTYPE;
+  if (M < 0 || N < 0 || K < 0 || E <= 0 || M > 0x7fffffffLL || ldx < K || ldy < N) return MOE_ERR_SHAPE;
+  if (!m_sizes) return MOE_ERR_NULL;
+  if (N == 0 || K == 0) return MOE_OK;
+  if (!w || (M > 0 && (!x || !dy))) return MOE_ERR_NULL;
+  if (M == 0) return cuda_status(cudaMemsetAsync(w, 0, (size_t)E * N * K * dtype_size(dtype), (cudaStream_t)stream));
+  if (!device_is_sm100()) return MOE_ERR_DEVICE;
+  const int path = g_path.load(std::memory_order_relaxed);
+  if (path == MOE_PATH_SIMT || ldx % 8 || ldy % 8 || !tc_eligible(2, x, dy, w, M, N, K, E, dtype, dtype)) return MOE_ERR_UNSUPPORTED;
+  return tc_grouped_gemm_dw_strided(x, ldx, dy, ldy, m_sizes, msd == MOE_I64, w, M, N, K, E, dtype, ws, ws_bytes,
+                                    (cudaStream_t)stream);
 }
 
 static int run_scattered(int which, const void* x, const void* w, const void* group_sizes, int msd,

@@ -44,6 +44,10 @@ struct GemmParams {
   const int* weight_index = nullptr;  // weight slice of each group (null: group e uses slice e)
   int* tile_counter = nullptr;  // work items are drawn from this counter (zeroed by build_group_maps_kernel); null: round-robin
   int stages = 0;               // CTA-pair forward / dX: depth of the operand ring
+  int ld_out = 0;               // single-CTA forward / dX: row pitch of the output (0: N)
+  float alpha[2] = {1.f, 1.f};  // single-CTA forward / dX: factors of the columns before / from b_split on
+  int scaled = 0;               //   (applied to the fp32 accumulator, when set)
+  int b_split = 0;              // single-CTA forward: columns taken from the first weight (0: there is one weight)
   int staged = 0;               // CTA-pair forward / dX: 16-bit output that may leave by TMA
   const int* row_index = nullptr;  // gathered forms: sorted row r reads row row_index[r] / index_div of the token tensor
   int index_div = 1;
@@ -152,9 +156,10 @@ __device__ __forceinline__ uint32_t pack2<__half>(float a, float b) {
 
 template <typename T>
 __device__ __forceinline__ void store_row_chunk16(T* dst, const uint32_t (&acc)[32], int ncols, bool vec) {
-  if (vec && ncols == 32) {
+  if (vec && (ncols & 7) == 0) {
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
+      if (8 * i >= ncols) break;
       uint4 v;
       v.x = pack2<T>(__uint_as_float(acc[8 * i + 0]), __uint_as_float(acc[8 * i + 1]));
       v.y = pack2<T>(__uint_as_float(acc[8 * i + 2]), __uint_as_float(acc[8 * i + 3]));
@@ -191,7 +196,7 @@ __device__ __forceinline__ void store_acc(void* out, int dtype_out, int64_t dst_
 template <int BN, bool B_MN>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
 tc_fwd_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
-              const GemmParams p) {
+              const GemmParams p, const __grid_constant__ CUtensorMap tmap_b2) {
   constexpr int B_CHUNKS = (BN + 63) / 64;  // 64-wide chunks of an MN-major B tile
   constexpr int B_STAGE_BYTES = B_MN ? B_CHUNKS * BK * 128 : (BN < 8 ? 8 : BN) * BK * 2;
   constexpr int STAGE_BYTES = A_STAGE_BYTES + ((B_STAGE_BYTES + 1023) & ~1023);
@@ -249,10 +254,13 @@ tc_fwd_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant_
           if (!mbar_wait(&ctl->empty[s], ph ^ 1, abort_flag, W_EMPTY)) { ok = false; break; }
           uint8_t* sa = smem + s * STAGE_BYTES;
           uint8_t* sb = sa + A_STAGE_BYTES;
-          mbar_expect_tx(&ctl->full[s], A_STAGE_BYTES + B_STAGE_BYTES);
+          // two weights side by side (b_split): their boxes hold exactly their rows, multiples of 8, so the second
+          // starts on a whole swizzle atom; the columns from p.N to BN multiply what the stage held before, unstored
+          mbar_expect_tx(&ctl->full[s], A_STAGE_BYTES + (p.b_split ? p.N * (BK * 2) : B_STAGE_BYTES));
           tma_load_2d(sa, &tmap_a, &ctl->full[s], kb * BK, m0);
           if constexpr (!B_MN) {
             tma_load_3d(sb, &tmap_b, &ctl->full[s], kb * BK, n0, e);
+            if (p.b_split) tma_load_3d(sb + p.b_split * (BK * 2), &tmap_b2, &ctl->full[s], kb * BK, 0, e);
           } else {
 #pragma unroll
             for (int c = 0; c < B_CHUNKS; ++c)
@@ -297,7 +305,8 @@ tc_fwd_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant_
     // ------------------------------ epilogue ------------------------------
     const int quarter = warp & 3;  // TMEM lanes this warp may read: [32*quarter, +32)
     const int row_in_tile = quarter * 32 + lane;
-    const bool vec = ((p.N * (int)dtype_size(p.dtype_out)) % 16 == 0) && ((reinterpret_cast<uintptr_t>(p.out) & 15) == 0);
+    const int ld = p.ld_out ? p.ld_out : p.N;
+    const bool vec = ((ld * (int)dtype_size(p.dtype_out)) % 16 == 0) && ((reinterpret_cast<uintptr_t>(p.out) & 15) == 0);
     uint32_t acc_it = 0;
     bool ok = true;
     for (int64_t tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x, ++acc_it) {
@@ -322,7 +331,12 @@ tc_fwd_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant_
         tmem_ld_wait();
         if (row_ok) {
           const int ncols = min(32, p.N - (n0 + c));
-          store_acc(p.out, p.dtype_out, grow * p.N + n0 + c, v, ncols, vec);
+          if (p.scaled) {
+#pragma unroll
+            for (int i = 0; i < 32; ++i)
+              v[i] = __float_as_uint(__uint_as_float(v[i]) * (p.b_split && n0 + c + i >= p.b_split ? p.alpha[1] : p.alpha[0]));
+          }
+          store_acc(p.out, p.dtype_out, grow * ld + n0 + c, v, ncols, vec);
         }
       }
       tc_fence_before_sync();
@@ -855,7 +869,7 @@ static int launch_pair_threads(void (*kernel)(KArgs...), int grid, int threads, 
 // dW on tensor cores: per-expert maps are built into `ws`, then one GEMM launch.
 static int dw_grouped_gemm(const void* x, const void* dy, const void* m_sizes, int ms64, void* out, int64_t M, int N,
                            int K, int E, int dtype_in, int dtype_out, void* ws, size_t ws_bytes, cudaStream_t stream,
-                           bool single_cta) {
+                           bool single_cta, int64_t ldx = 0, int64_t ldy = 0) {
   using namespace tc;
   if (!ws_usable(ws, ws_bytes, E)) return MOE_ERR_WORKSPACE;
   GemmParams p;
@@ -867,8 +881,8 @@ static int dw_grouped_gemm(const void* x, const void* dy, const void* m_sizes, i
   int st;
   GroupMapTemplates tm;
   tm.mask = (1 << GM_DY) | (1 << GM_X);
-  if ((st = make_map(&tm.t[GM_DY], dtype_in, dy, (uint64_t)N, (uint64_t)M, 0, BK)) != MOE_OK) return st;
-  if ((st = make_map(&tm.t[GM_X], dtype_in, x, (uint64_t)K, (uint64_t)M, 0, BK)) != MOE_OK) return st;
+  if ((st = make_map(&tm.t[GM_DY], dtype_in, dy, (uint64_t)N, (uint64_t)M, 0, BK, (uint64_t)ldy)) != MOE_OK) return st;
+  if ((st = make_map(&tm.t[GM_X], dtype_in, x, (uint64_t)K, (uint64_t)M, 0, BK, (uint64_t)ldx)) != MOE_OK) return st;
   const int gm_smem = 8 * 128 + 2 * (E + 1) * 4 + 128;
   build_group_maps_kernel<<<(E + 7) / 8, 256, gm_smem, stream>>>(tm, m_sizes, ms64, E, M, reinterpret_cast<CUtensorMap*>(ws),
                                                                  ws_counter(ws, E));
@@ -917,6 +931,69 @@ static int dw_grouped_gemm(const void* x, const void* dy, const void* m_sizes, i
   return launch_status();
 }
 
+// What the LoRA projections add to the single-CTA forward / dX: factors, an output pitch, a second weight.
+struct SingleExtra {
+  float alpha[2] = {1.f, 1.f};
+  const void* b2 = nullptr;  // forward: N = n1 + n2 columns, the first n1 from b, the others from b2
+  int n1 = 0;
+  int ld_out = 0;
+};
+
+static int single_grouped_gemm(int which, const void* a, const void* b, const void* m_sizes, int ms64, void* out,
+                               int64_t M, int N, int K, int E, int dtype_in, int dtype_out, cudaStream_t stream,
+                               const SingleExtra& x) {
+  using namespace tc;
+  if (which != 0 && which != 1) return MOE_ERR_UNSUPPORTED;
+  GemmParams p;
+  p.m_sizes = m_sizes; p.out = out; p.M = M; p.N = N; p.K = K; p.E = E; p.ms64 = ms64; p.dtype_out = dtype_out;
+  p.alpha[0] = x.alpha[0]; p.alpha[1] = x.alpha[1];
+  p.scaled = x.alpha[0] != 1.f || x.alpha[1] != 1.f;
+  p.ld_out = x.ld_out;
+  p.b_split = x.b2 ? x.n1 : 0;
+  const int fmt = dtype_in == MOE_BF16 ? 1 : 0;
+  const int grid = sm_count();
+  CUtensorMap ma, mb, mb2;
+  int st;
+  // narrowest accumulator that covers N: thin outputs (LoRA down-projections) do not pay for 128 columns
+  const int bn = N > 128 ? 256 : N > 64 ? 128 : N > 32 ? 64 : N > 16 ? 32 : 16;
+  if (p.b_split && (which != 0 || N > 256)) return MOE_ERR_UNSUPPORTED;  // one column tile
+  if ((st = make_map(&ma, dtype_in, a, (uint64_t)K, (uint64_t)M, 0, BM)) != MOE_OK) return st;
+  const int n1 = p.b_split ? p.b_split : N;
+  if (which == 0) st = make_map(&mb, dtype_in, b, (uint64_t)K, (uint64_t)n1, (uint64_t)E, (uint32_t)(p.b_split ? n1 : bn));
+  else st = make_map(&mb, dtype_in, b, (uint64_t)N, (uint64_t)K, (uint64_t)E, BK);
+  if (st != MOE_OK) return st;
+  mb2 = mb;
+  if (p.b_split && (st = make_map(&mb2, dtype_in, x.b2, (uint64_t)K, (uint64_t)(N - n1), (uint64_t)E, (uint32_t)(N - n1))) != MOE_OK)
+    return st;
+  p.idesc = make_idesc(fmt, 0, which == 1, BM, bn);
+#define MOE_TC_LAUNCH(BN_, BMN_)                                                              \
+  do {                                                                                        \
+    const int bytes = smem_bytes_for<BN_>(E, 2);                                              \
+    if (bytes > SMEM_LIMIT) return MOE_ERR_UNSUPPORTED;                                       \
+    if ((st = set_smem(tc_fwd_kernel<BN_, BMN_>, bytes)) != MOE_OK) return st;                \
+    tc_fwd_kernel<BN_, BMN_><<<grid, NUM_THREADS, bytes, stream>>>(ma, mb, p, mb2);           \
+  } while (0)
+  if (which == 0) {
+    switch (bn) {
+      case 256: MOE_TC_LAUNCH(256, false); break;
+      case 128: MOE_TC_LAUNCH(128, false); break;
+      case 64: MOE_TC_LAUNCH(64, false); break;
+      case 32: MOE_TC_LAUNCH(32, false); break;
+      default: MOE_TC_LAUNCH(16, false); break;
+    }
+  } else {
+    switch (bn) {
+      case 256: MOE_TC_LAUNCH(256, true); break;
+      case 128: MOE_TC_LAUNCH(128, true); break;
+      case 64: MOE_TC_LAUNCH(64, true); break;
+      case 32: MOE_TC_LAUNCH(32, true); break;
+      default: MOE_TC_LAUNCH(16, true); break;
+    }
+  }
+#undef MOE_TC_LAUNCH
+  return launch_status();
+}
+
 // which: 0 forward, 1 dX, 2 dW (a = x, b = dy).  single_cta selects the one-CTA kernels.
 int tc_grouped_gemm(int which, const void* a, const void* b, const void* m_sizes, int ms64, void* out,
                     int64_t M, int N, int K, int E, int dtype_in, int dtype_out, void* ws, size_t ws_bytes,
@@ -932,48 +1009,8 @@ int tc_grouped_gemm(int which, const void* a, const void* b, const void* m_sizes
     const PairOperand op{a, b, K, 0};
     if (pair_ok) return pair_grouped_gemm(which, &op, 1, m_sizes, ms64, out, M, N, E, dtype_in, dtype_out, ws, ws_bytes, stream);
   }
-  GemmParams p;
-  p.m_sizes = m_sizes; p.out = out; p.M = M; p.N = N; p.K = K; p.E = E; p.ms64 = ms64; p.dtype_out = dtype_out;
-  const int fmt = dtype_in == MOE_BF16 ? 1 : 0;
-  const int grid = sm_count();
-  CUtensorMap ma, mb;
-  int st;
-  if (which == 0 || which == 1) {
-    // narrowest accumulator that covers N: thin outputs (LoRA down-projections) do not pay for 128 columns
-    const int bn = N > 128 ? 256 : N > 64 ? 128 : N > 32 ? 64 : N > 16 ? 32 : 16;
-    if ((st = make_map(&ma, dtype_in, a, (uint64_t)K, (uint64_t)M, 0, BM)) != MOE_OK) return st;
-    if (which == 0) st = make_map(&mb, dtype_in, b, (uint64_t)K, (uint64_t)N, (uint64_t)E, (uint32_t)bn);
-    else st = make_map(&mb, dtype_in, b, (uint64_t)N, (uint64_t)K, (uint64_t)E, BK);
-    if (st != MOE_OK) return st;
-    p.idesc = make_idesc(fmt, 0, which == 1, BM, bn);
-#define MOE_TC_LAUNCH(BN_, BMN_)                                                              \
-  do {                                                                                        \
-    const int bytes = smem_bytes_for<BN_>(E, 2);                                              \
-    if (bytes > SMEM_LIMIT) return MOE_ERR_UNSUPPORTED;                                       \
-    if ((st = set_smem(tc_fwd_kernel<BN_, BMN_>, bytes)) != MOE_OK) return st;                \
-    tc_fwd_kernel<BN_, BMN_><<<grid, NUM_THREADS, bytes, stream>>>(ma, mb, p);                \
-  } while (0)
-    if (which == 0) {
-      switch (bn) {
-        case 256: MOE_TC_LAUNCH(256, false); break;
-        case 128: MOE_TC_LAUNCH(128, false); break;
-        case 64: MOE_TC_LAUNCH(64, false); break;
-        case 32: MOE_TC_LAUNCH(32, false); break;
-        default: MOE_TC_LAUNCH(16, false); break;
-      }
-    } else {
-      switch (bn) {
-        case 256: MOE_TC_LAUNCH(256, true); break;
-        case 128: MOE_TC_LAUNCH(128, true); break;
-        case 64: MOE_TC_LAUNCH(64, true); break;
-        case 32: MOE_TC_LAUNCH(32, true); break;
-        default: MOE_TC_LAUNCH(16, true); break;
-      }
-    }
-#undef MOE_TC_LAUNCH
-    return launch_status();
-  }
-  return MOE_ERR_UNSUPPORTED;
+  const SingleExtra plain;
+  return single_grouped_gemm(which, a, b, m_sizes, ms64, out, M, N, K, E, dtype_in, dtype_out, stream, plain);
 }
 
 // h = silu(x w_gate^T) * (x w_up^T) per expert in one launch (pair_fwd_kernel<false, true>).
@@ -1030,6 +1067,33 @@ int tc_grouped_gemm_scattered(int which, const void* a, const void* b, const voi
   const PairOperand op{a, b, K, 0};
   return pair_grouped_gemm(which, &op, 1, group_sizes, ms64, out_template, M, N, G, dtype_in, dtype_out, ws, ws_bytes,
                            stream, weight_index, n_weights, out_ptrs);
+}
+
+// y = sum_i x_i W_i^T (which = 0) or sum_i x_i W_i (which = 1), the contractions of n operand pairs in one accumulator.
+int tc_grouped_gemm_sum(int which, int n, const void* const* x, const int64_t* ldx, const void* const* w, const int* K,
+                        const void* m_sizes, int ms64, void* out, int64_t M, int N, int E, int dtype, cudaStream_t stream) {
+  bind_context_once();
+  PairOperand ops[tc::PAIR_MAX_SEGS];
+  for (int i = 0; i < n; ++i) ops[i] = PairOperand{x[i], w[i], K[i], ldx[i]};
+  return pair_grouped_gemm(which, ops, n, m_sizes, ms64, out, M, N, E, dtype, dtype, nullptr, 0, stream);
+}
+
+// LoRA projections: the single-CTA forward (one or two weights side by side) / dX with factors and an output pitch.
+int tc_lora_project(int which, const void* x, const void* a0, int n0, float s0, const void* a1, int n1, float s1,
+                    const void* m_sizes, int ms64, void* out, int ld_out, int64_t M, int K, int E, int dtype,
+                    cudaStream_t stream) {
+  bind_context_once();
+  SingleExtra ex;
+  ex.alpha[0] = s0; ex.alpha[1] = a1 ? s1 : s0;
+  ex.b2 = a1; ex.n1 = n0; ex.ld_out = ld_out;
+  return single_grouped_gemm(which, x, a0, m_sizes, ms64, out, M, n0 + (a1 ? n1 : 0), K, E, dtype, dtype, stream, ex);
+}
+
+int tc_grouped_gemm_dw_strided(const void* x, int64_t ldx, const void* dy, int64_t ldy, const void* m_sizes, int ms64,
+                               void* out, int64_t M, int N, int K, int E, int dtype, void* ws, size_t ws_bytes,
+                               cudaStream_t stream) {
+  bind_context_once();
+  return dw_grouped_gemm(x, dy, m_sizes, ms64, out, M, N, K, E, dtype, dtype, ws, ws_bytes, stream, false, ldx, ldy);
 }
 
 bool tc_nf4_eligible(const void* x, const void* packed, const void* absmax, const void* out, int64_t M, int N, int K,

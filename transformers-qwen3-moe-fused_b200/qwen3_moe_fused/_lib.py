@@ -7,7 +7,7 @@ from __future__ import annotations
 
 import ctypes
 import os
-from ctypes import c_char_p, c_int, c_int64, c_size_t, c_void_p
+from ctypes import c_char_p, c_float, c_int, c_int64, c_size_t, c_void_p
 from pathlib import Path
 
 import torch
@@ -22,7 +22,7 @@ _INT_CODES = {torch.int32: I32, torch.int64: I64}
 _LIB_PATH = Path(__file__).resolve().parent / "libmoe_b200.so"
 
 # name -> (restype, argtypes); mirrors include/moe_b200.h one to one
-_P, _I, _L, _Z = c_void_p, c_int, c_int64, c_size_t
+_P, _I, _L, _Z, _F = c_void_p, c_int, c_int64, c_size_t, c_float
 SIGNATURES = {
     "moe_b200_version": (_I, []),
     "moe_status_string": (c_char_p, [_I]),
@@ -37,6 +37,9 @@ SIGNATURES = {
     "moe_grouped_gemm_fwd": (_I, [_P, _P, _P, _I, _P, _L, _I, _I, _I, _I, _I, _P, _Z, _P]),
     "moe_grouped_gemm_dx": (_I, [_P, _P, _P, _I, _P, _L, _I, _I, _I, _I, _I, _P, _Z, _P]),
     "moe_grouped_gemm_dw": (_I, [_P, _P, _P, _I, _P, _L, _I, _I, _I, _I, _I, _P, _Z, _P]),
+    "moe_grouped_gemm_sum": (_I, [_I, _I, _P, _P, _P, _P, _P, _I, _P, _L, _I, _I, _I, _P]),
+    "moe_lora_project": (_I, [_I, _P, _P, _I, _F, _P, _I, _F, _P, _I, _P, _L, _L, _I, _I, _I, _P]),
+    "moe_grouped_gemm_dw_strided": (_I, [_P, _L, _P, _L, _P, _I, _P, _L, _I, _I, _I, _I, _P, _Z, _P]),
     "moe_gate_up_silu_fwd": (_I, [_P, _P, _P, _P, _I, _P, _L, _I, _I, _I, _I, _P, _Z, _P]),
     "moe_gate_up_silu_fwd_gather": (_I, [_P, _L, _P, _I, _P, _P, _P, _I, _P, _L, _I, _I, _I, _I, _P, _Z, _P]),
     "moe_grouped_gemm_fwd_gather": (_I, [_P, _L, _P, _I, _P, _P, _I, _P, _L, _I, _I, _I, _I, _I, _P, _Z, _P]),
