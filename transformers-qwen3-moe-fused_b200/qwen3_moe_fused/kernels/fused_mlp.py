@@ -1,4 +1,5 @@
-"""Gate projection + up projection + SiLU-mul of the expert MLP in one kernel (inference).
+"""Gate projection + up projection + SiLU-mul of the expert MLP: one kernel for inference, one autograd
+function for training.
 
 What the reference block computes with two `moe_fused_linear` calls and `F.silu(gate_h) * up_h`
 (qwen3_moe_fused/modular_qwen3_moe_fused.py:105-108), with the same rounding points, so the
@@ -9,8 +10,11 @@ from typing import Optional
 import torch
 
 from .. import _lib
+from ..grouped_gemm.backward_dw import grouped_gemm_backward_dw
 from ..grouped_gemm.forward import grouped_gemm_forward
-from .silu_mul import silu_mul_forward
+from ..grouped_gemm.forward_transposed import grouped_gemm_forward_transposed
+from ..grouped_gemm.lora import eligible, grouped_gemm_sum
+from .silu_mul import silu_mul_backward, silu_mul_forward
 
 
 @torch.no_grad()
@@ -59,3 +63,36 @@ def gate_up_silu_forward(x: torch.Tensor, gate_proj: torch.Tensor, up_proj: torc
             return h
     # shapes / dtypes the fused kernel does not cover: the three kernels it stands for
     return silu_mul_forward(grouped_gemm_forward(x, gate_proj, m_sizes), grouped_gemm_forward(x, up_proj, m_sizes))
+
+
+class GateUpSilu(torch.autograd.Function):
+    """h = silu(x gate^T) * (x up^T) with rows of x sorted by expert.  Same forward as two `moe_fused_linear` and
+    `silu_mul`; the backward contracts both gradients with their weights in one launch (dx = de gate + dg up in one
+    fp32 accumulator) instead of writing two partial dx and adding them."""
+
+    @staticmethod
+    def forward(ctx, x, gate_proj, up_proj, m_sizes):
+        e = grouped_gemm_forward(x, gate_proj, m_sizes)
+        g = grouped_gemm_forward(x, up_proj, m_sizes)
+        ctx.save_for_backward(x, gate_proj, up_proj, m_sizes, e, g)
+        return silu_mul_forward(e, g)
+
+    @staticmethod
+    def backward(ctx, dh):
+        x, gate_proj, up_proj, m_sizes, e, g = ctx.saved_tensors
+        de, dg = silu_mul_backward(dh.contiguous(), e, g)
+        dx = d_gate = d_up = None
+        if ctx.needs_input_grad[0]:
+            if eligible(de, (gate_proj, up_proj), m_sizes):
+                dx = grouped_gemm_sum(((de, gate_proj), (dg, up_proj)), m_sizes, True)
+            if dx is None:
+                dx = grouped_gemm_forward_transposed(de, gate_proj, m_sizes, x.dtype)
+                dx += grouped_gemm_forward_transposed(dg, up_proj, m_sizes, x.dtype)
+        if ctx.needs_input_grad[1]:
+            d_gate = grouped_gemm_backward_dw(x, de, m_sizes, gate_proj.dtype)
+        if ctx.needs_input_grad[2]:
+            d_up = grouped_gemm_backward_dw(x, dg, m_sizes, up_proj.dtype)
+        return dx, d_gate, d_up, None
+
+
+gate_up_silu = GateUpSilu.apply

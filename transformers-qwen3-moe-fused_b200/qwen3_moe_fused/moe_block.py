@@ -16,10 +16,9 @@ import torch
 from torch import nn
 
 from .functional import moe_fused_linear
-from .kernels.fused_mlp import gate_up_silu_forward
+from .kernels.fused_mlp import gate_up_silu, gate_up_silu_forward
 from .kernels.indexing import get_expert_counts_and_idx
 from .kernels.routing import combine, gather_rows, softmax_topk_autograd
-from .kernels.silu_mul import silu_mul
 
 
 # The inference path can feed gate / up straight from the token tensor (TMA gather4 in the token load,
@@ -84,9 +83,7 @@ def moe_block_forward(hidden_states: torch.Tensor, gate_weight: torch.Tensor, ga
         h = gate_up_silu_forward(gather_rows(x.contiguous(), sort_idx, inv_sort_idx, k), gate_proj, up_proj, m_sizes)
     else:
         xs = gather_rows(x.contiguous(), sort_idx, inv_sort_idx, k)
-        gate_h = moe_fused_linear(xs, gate_proj, m_sizes)
-        up_h = moe_fused_linear(xs, up_proj, m_sizes)
-        h = silu_mul(gate_h, up_h)
+        h = gate_up_silu(xs, gate_proj, up_proj, m_sizes)
     y = moe_fused_linear(h, down_proj, m_sizes)
     out = combine(y, sort_idx, inv_sort_idx, routing_weights)
     return out.view(B, S, H), router_logits
