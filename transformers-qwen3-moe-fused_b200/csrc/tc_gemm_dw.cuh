@@ -27,7 +27,7 @@ namespace moe {
 namespace tc {
 
 struct GroupMapTemplates {
-  static constexpr int MAX = 2;
+  static constexpr int MAX = 3;  // (of which two are in use; callers size their workspace by three)
   CUtensorMap t[MAX];
   int mask;  // bit t set: slot t is derived for every expert
 };
