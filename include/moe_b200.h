@@ -244,6 +244,41 @@ int moe_expand_rows(const void* hidden, const int32_t* inv_sort_idx, int k, void
 int moe_combine(const void* y, const int32_t* inv_sort_idx, const void* weights, void* out,
                 int64_t T, int k, int H, int dtype, void* stream);
 
+/* The inference forward of the sparse MoE block after its router GEMM: router softmax + top-k, sort, expand, fused
+ * gate / up / SiLU-mul, down projection, weighted combine, enqueued by one call on scratch memory of
+ * moe_block_fwd_scratch_bytes bytes (0: sizes not supported), 256-byte aligned.  x (T, H), logits (T, E),
+ * w_gate / w_up (E, I, H), w_down (E, H, I), out (T, H), all of one 16-bit dtype and contiguous.
+ * MOE_ERR_UNSUPPORTED (nothing enqueued) where moe_gate_up_silu_fwd would not take the weights.
+ * Replaces qwen3_moe_fused/modular_qwen3_moe_fused.py:87-117. */
+size_t moe_block_fwd_scratch_bytes(int64_t T, int H, int I, int E, int k, int dtype);
+int moe_block_fwd(const void* x, const void* logits, const void* w_gate, const void* w_up, const void* w_down, void* out,
+                  int64_t T, int H, int I, int E, int k, int norm_topk, int dtype, void* scratch, size_t scratch_bytes,
+                  void* stream);
+
+/* The expert MLP with LoRA on dense 16-bit weights, gate / up / down in this order: forward and backward as one call
+ * each, built from moe_lora_project, moe_grouped_gemm_sum, moe_grouped_gemm_dw_strided and the SiLU-mul kernels (their
+ * conditions apply to every operand).  base (E, I, H), (E, I, H), (E, H, I); a (E, r, in), b (E, out, r).
+ * Forward: e, g, h (M, I), t_gu (M, r_gate + r_up), t_w (M, r_down), y (M, H) are written; all but h and y are what the
+ * backward needs.  Backward: e and g are overwritten; dh (M, I), d_gu, d_w (shaped like t_gu, t_w) are scratch; dx may
+ * be NULL (not wanted); ws as for moe_grouped_gemm_dw.
+ * Replaces qwen3_moe_fused/kernels/fast_lora.py:66-175. */
+typedef struct {
+  const void* base[3];
+  const void* a[3];
+  const void* b[3];
+  float scale[3];
+  int rank[3];
+} moe_lora_weights;
+typedef struct {
+  void* da[3];
+  void* db[3];
+} moe_lora_grads;
+int moe_lora_mlp_fwd(const moe_lora_weights* w, const void* x, const void* m_sizes, int msd, void* e, void* g, void* h,
+                     void* t_gu, void* t_w, void* y, int64_t M, int H, int I, int E, int dtype, void* stream);
+int moe_lora_mlp_bwd(const moe_lora_weights* w, const moe_lora_grads* grads, const void* dy, const void* x,
+                     const void* m_sizes, int msd, void* e, void* g, const void* t_gu, const void* t_w, void* dh, void* d_gu,
+                     void* d_w, void* dx, int64_t M, int H, int I, int E, int dtype, void* ws, size_t ws_bytes, void* stream);
+
 /* Backward of moe_combine in one pass: dy[inv_sort_idx[t*k+j], :] = weights[t,j] * dout[t,:] and
  * dweights[t,j] = <dout[t,:], y[inv_sort_idx[t*k+j], :]> (fp32 sums).  dy or dweights may be NULL (not wanted);
  * weights is read for dy, y for dweights.

@@ -31,3 +31,33 @@ def test_gate_up_silu_backward(cuda, H, I, frozen):
     # chains of at most six roundings one after the other, each at most 2^-8 of what it applies to: 2-norm over 2-norm
     for got, want in zip((h, *grads), (ref, *torch.autograd.grad(ref, [t for t in d if t.requires_grad], dh.double()))):
         assert (got.double() - want).norm() <= 6 * 2.0 ** -8 * want.norm()
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("T,E,k,H,I,norm", [(1, 128, 8, 256, 64, True), (3, 8, 8, 200, 72, False), (257, 5, 2, 64, 200, True),
+                                            (300, 128, 8, 520, 192, True)])
+def test_block_call_equals_composition(cuda, dtype, T, E, k, H, I, norm):
+    """Same kernels in the same order, so the same bits."""
+    from qwen3_moe_fused.functional import moe_fused_linear
+    from qwen3_moe_fused.kernels.fused_mlp import gate_up_silu_forward
+    from qwen3_moe_fused.kernels.indexing import get_expert_counts_and_idx
+    from qwen3_moe_fused.kernels.routing import combine, gather_rows
+    from qwen3_moe_fused.moe_block import _block_infer, moe_block_forward, route
+
+    gen = torch.Generator(device=cuda).manual_seed(T)
+    x, gw, gp, up, dp = ((torch.randn(*s, device=cuda, generator=gen) * 0.1).to(dtype)
+                         for s in ((T, H), (E, H), (E, I, H), (E, I, H), (E, H, I)))
+    with torch.no_grad():
+        logits = torch.nn.functional.linear(x, gw)
+        w, sel = route(logits, k, norm, dtype)
+        m_sizes, si, ii = get_expert_counts_and_idx(sel.view(T * k), E)
+        y = moe_fused_linear(gate_up_silu_forward(gather_rows(x, si, ii, k), gp, up, m_sizes), dp, m_sizes)
+        want = combine(y, si, ii, w)
+        assert torch.equal(_block_infer(x, logits, gp, up, dp, k, norm), want)
+        out, lg = moe_block_forward(x.view(1, T, H), gw, gp, up, dp, k, norm)
+        assert torch.equal(out.view(T, H), want) and torch.equal(lg, logits)
+        # an up projection that is not 16-byte aligned takes the composition
+        odd = torch.empty(up.numel() + 1, device=cuda, dtype=dtype)[1:].view_as(up).copy_(up)
+        assert _block_infer(x, logits, gp, odd, dp, k, norm) is None
+        out, _ = moe_block_forward(x.view(1, T, H), gw, gp, odd, dp, k, norm)
+        assert torch.allclose(out.view(T, H).float(), want.float(), rtol=2e-2, atol=2e-3 * want.float().abs().max().item())

@@ -56,6 +56,10 @@ SIGNATURES = {
     "moe_expand_rows": (_I, [_P, _P, _I, _P, _L, _I, _I, _P]),
     "moe_combine": (_I, [_P, _P, _P, _P, _L, _I, _I, _I, _P]),
     "moe_combine_bwd": (_I, [_P, _P, _P, _P, _P, _P, _L, _I, _I, _I, _P]),
+    "moe_block_fwd_scratch_bytes": (_Z, [_L, _I, _I, _I, _I, _I]),
+    "moe_block_fwd": (_I, [_P, _P, _P, _P, _P, _P, _L, _I, _I, _I, _I, _I, _I, _P, _Z, _P]),
+    "moe_lora_mlp_fwd": (_I, [_P, _P, _P, _I, _P, _P, _P, _P, _P, _P, _L, _I, _I, _I, _I, _P]),
+    "moe_lora_mlp_bwd": (_I, [_P, _P, _P, _P, _P, _I, _P, _P, _P, _P, _P, _P, _P, _P, _L, _I, _I, _I, _I, _P, _Z, _P]),
     "moe_ep_plan": (_I, [_P, _I, _I, _I, _I, _I, _P, _P, _P, _P, _P, _P, _P, _P, _P]),
     "moe_ep_push_rows": (_I, [_P, _L, _L, _P, _I, _I, _P, _P, _I, _P, _I, _I, _P, _P]),
     "moe_ep_token_positions": (_I, [_P, _I, _L, _I, _I, _I, _P, _P, _P]),
@@ -68,6 +72,18 @@ SIGNATURES = {
     "moe_debug_read_late_values": (_I, [_P]),
     "moe_debug_last_detail": (c_char_p, []),
 }
+
+
+
+class LoraWeights(ctypes.Structure):
+    """moe_lora_weights; entries 0, 1, 2 are gate, up, down."""
+    _fields_ = [("base", c_void_p * 3), ("a", c_void_p * 3), ("b", c_void_p * 3), ("scale", c_float * 3), ("rank", c_int * 3)]
+
+
+class LoraGrads(ctypes.Structure):
+    """moe_lora_grads."""
+    _fields_ = [("da", c_void_p * 3), ("db", c_void_p * 3)]
+
 
 _lib = None
 

@@ -16,15 +16,17 @@ Differences in how the same quantities are computed:
   * on dense 16-bit weights every `base product + s * (t B)` is one launch that contracts both operand
     pairs into one accumulator (dx: four pairs), with s applied to the fp32 accumulator of the thin factor.
 """
+import ctypes
 import math
 
 import torch
 
+from .. import _lib
 from ..grouped_gemm.backward_dw import grouped_gemm_backward_dw
 from ..grouped_gemm.forward import grouped_gemm_forward
 from ..grouped_gemm.forward_4bit import grouped_gemm_forward_4bit, grouped_gemm_forward_transposed_4bit
 from ..grouped_gemm.forward_transposed import grouped_gemm_forward_transposed
-from ..grouped_gemm.lora import eligible, grouped_gemm_dw_strided, grouped_gemm_sum, lora_project
+from ..grouped_gemm.lora import eligible
 from ..quantize.nf4 import dequantize_4bit
 from .silu_mul import silu_mul_backward_inplace, silu_mul_forward
 
@@ -56,6 +58,11 @@ def _fits_fused(x, base, quant, adapters, scales, m_sizes) -> bool:
         Bg.shape == (E, I, rg) and Bu.shape == (E, I, ru) and Bw.shape == (E, H, rw)
 
 
+def _lora_weights(base, a, b, scales) -> _lib.LoraWeights:
+    ptrs = lambda ts: (ctypes.c_void_p * 3)(*(t.data_ptr() for t in ts))
+    return _lib.LoraWeights(ptrs(base), ptrs(a), ptrs(b), (ctypes.c_float * 3)(*scales), (ctypes.c_int * 3)(*(t.shape[1] for t in a)))
+
+
 class FastLora(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, Gq, Gqs, Ag, Bg, Sg, Uq, Uqs, Au, Bu, Su, Wq, Wqs, Aw, Bw, Sw, m_sizes):
@@ -71,16 +78,18 @@ class FastLora(torch.autograd.Function):
 
         ctx.fused = _fits_fused(x, (Gq, Uq, Wq), (Gqs, Uqs, Wqs), (Ag, Bg, Au, Bu, Aw, Bw), (Sg, Su, Sw), m_sizes)
         if ctx.fused:
-            M, rg, rw = x.shape[0], Ag.shape[1], Aw.shape[1]
-            # thin factors of the LoRA products, already scaled: gate and up side by side (x is read once), down
-            t_gu = torch.empty((M, rg + Au.shape[1]), device=x.device, dtype=dt)
-            lora_project(x, Ag, Sg, m_sizes, t_gu, Au, Su)
-            e = grouped_gemm_sum(((x, Gq), (t_gu[:, :rg], Bg)), m_sizes, False)
-            g = grouped_gemm_sum(((x, Uq), (t_gu[:, rg:], Bu)), m_sizes, False)
-            h = silu_mul_forward(e, g)
-            t_w = torch.empty((M, rw), device=x.device, dtype=dt)
-            lora_project(h, Aw, Sw, m_sizes, t_w)
-            y = grouped_gemm_sum(((h, Wq), (t_w, Bw)), m_sizes, False)
+            M, H, (E, I) = x.shape[0], x.shape[1], Gq.shape[:2]
+            # t_gu, t_w: the thin factors s x A^T of the LoRA products, gate and up side by side
+            e, g, h, t_gu, t_w, y = (torch.empty((M, n), device=x.device, dtype=dt)
+                                     for n in (I, I, I, Ag.shape[1] + Au.shape[1], Aw.shape[1], H))
+            w = _lora_weights((Gq, Uq, Wq), (Ag, Au, Aw), (Bg, Bu, Bw), (Sg, Su, Sw))
+            ms = _lib.as_index_tensor(m_sizes)
+            with torch.cuda.device(x.device):
+                status = _lib.load().moe_lora_mlp_fwd(
+                    ctypes.addressof(w), x.data_ptr(), ms.data_ptr(), _lib.int_code(ms.dtype), e.data_ptr(), g.data_ptr(),
+                    h.data_ptr(), t_gu.data_ptr(), t_w.data_ptr(), y.data_ptr(), M, H, I, E, _lib.float_code(dt),
+                    _lib.stream_ptr(x.device))
+            _lib.check(status, "moe_lora_mlp_fwd")
             ctx.custom_saved_tensors = (Gq, Gqs, Sg, Uq, Uqs, Su, Wq, Wqs, Sw, m_sizes)
             ctx.save_for_backward(x, Ag, Bg, Au, Bu, Aw, Bw, e, g, t_gu, t_w)
             return y
@@ -161,30 +170,26 @@ class FastLora(torch.autograd.Function):
     def _backward_fused(ctx, dy):
         Gq, _, Sg, Uq, _, Su, Wq, _, Sw, m_sizes = ctx.custom_saved_tensors
         x, Ag, Bg, Au, Bu, Aw, Bw, e, g, t_gu, t_w = ctx.saved_tensors
-        rg = Ag.shape[1]
         dy = dy.contiguous().to(x.dtype)
         if dy.data_ptr() % 16:
             dy = dy.clone()
-
-        d_w = torch.empty_like(t_w)  # s dy B
-        lora_project(dy, Bw, Sw, m_sizes, d_w, transposed=True)
-        dh = grouped_gemm_sum(((dy, Wq), (d_w, Aw)), m_sizes, True)
-        # dh, e, g become h, de, dg
-        silu_mul_backward_inplace(dh, e, g)
-        h, de, dg = dh, e, g
-        del dh, e, g
-        dAw = grouped_gemm_dw_strided(h, d_w, m_sizes)
-        dBw = grouped_gemm_dw_strided(t_w, dy, m_sizes)
-        d_gu = torch.empty_like(t_gu)  # [s de B | s dg B]
-        lora_project(de, Bg, Sg, m_sizes, d_gu[:, :rg], transposed=True)
-        lora_project(dg, Bu, Su, m_sizes, d_gu[:, rg:], transposed=True)
-        dAg = grouped_gemm_dw_strided(x, d_gu[:, :rg], m_sizes)
-        dAu = grouped_gemm_dw_strided(x, d_gu[:, rg:], m_sizes)
-        dBg = grouped_gemm_dw_strided(t_gu[:, :rg], de, m_sizes)
-        dBu = grouped_gemm_dw_strided(t_gu[:, rg:], dg, m_sizes)
-        dx = None
-        if ctx.needs_input_grad[0]:
-            dx = grouped_gemm_sum(((de, Gq), (d_gu[:, :rg], Ag), (dg, Uq), (d_gu[:, rg:], Au)), m_sizes, True)
+        M, H, (E, I) = x.shape[0], x.shape[1], Gq.shape[:2]
+        code = _lib.float_code(x.dtype)
+        dAg, dAu, dAw, dBg, dBu, dBw, d_gu, d_w = (torch.empty_like(t) for t in (Ag, Au, Aw, Bg, Bu, Bw, t_gu, t_w))
+        dh = torch.empty_like(e)
+        dx = torch.empty_like(x) if ctx.needs_input_grad[0] else None
+        w = _lora_weights((Gq, Uq, Wq), (Ag, Au, Aw), (Bg, Bu, Bw), (Sg, Su, Sw))
+        grads = _lib.LoraGrads((ctypes.c_void_p * 3)(dAg.data_ptr(), dAu.data_ptr(), dAw.data_ptr()),
+                               (ctypes.c_void_p * 3)(dBg.data_ptr(), dBu.data_ptr(), dBw.data_ptr()))
+        ms = _lib.as_index_tensor(m_sizes)
+        lib = _lib.load()
+        ws_ptr, ws_bytes = _lib.workspace(x.device, lib.moe_grouped_gemm_workspace_bytes(2, M, H, I, E))
+        with torch.cuda.device(x.device):
+            status = lib.moe_lora_mlp_bwd(  # overwrites dh, e, g with h, de, dg
+                ctypes.addressof(w), ctypes.addressof(grads), dy.data_ptr(), x.data_ptr(), ms.data_ptr(), _lib.int_code(ms.dtype),
+                e.data_ptr(), g.data_ptr(), t_gu.data_ptr(), t_w.data_ptr(), dh.data_ptr(), d_gu.data_ptr(), d_w.data_ptr(),
+                _lib.ptr(dx), M, H, I, E, code, ws_ptr, ws_bytes, _lib.stream_ptr(x.device))
+        _lib.check(status, "moe_lora_mlp_bwd")
         return (dx, None, None, dAg, dBg, None, None, None, dAu, dBu, None, None, None, dAw, dBw, None, None)
 
 

@@ -15,6 +15,7 @@ from typing import Optional
 import torch
 from torch import nn
 
+from . import _lib
 from .functional import moe_fused_linear
 from .kernels.fused_mlp import gate_up_silu, gate_up_silu_forward
 from .kernels.indexing import get_expert_counts_and_idx
@@ -61,6 +62,35 @@ def route(router_logits: torch.Tensor, num_selected: int, norm_topk_prob: bool, 
     return softmax_topk_autograd(router_logits.contiguous(), num_selected, norm_topk_prob, dtype)
 
 
+def _block_infer(x, router_logits, gate_proj, up_proj, down_proj, k: int, norm_topk_prob: bool) -> Optional[torch.Tensor]:
+    """The block after its router GEMM as one call into the library (the same kernels in the same order as the
+    composition in `moe_block_forward`); None where that composition has to decide: other dtypes, layouts, extents."""
+    T, H = x.shape
+    ts = (x, router_logits, gate_proj, up_proj, down_proj)
+    if x.dtype not in (torch.bfloat16, torch.float16) or not x.is_cuda or gate_proj.ndim != 3:
+        return None
+    E, I = gate_proj.shape[0], gate_proj.shape[1]
+    if any(t.dtype != x.dtype or t.device != x.device or not t.is_contiguous() for t in ts) or \
+            gate_proj.shape != (E, I, H) or up_proj.shape != (E, I, H) or down_proj.shape != (E, H, I) or router_logits.shape != (T, E):
+        return None
+    lib = _lib.load()
+    code = _lib.float_code(x.dtype)
+    nbytes = lib.moe_block_fwd_scratch_bytes(T, H, I, E, k, code)
+    if nbytes == 0:
+        return None
+    with torch.cuda.device(x.device):
+        scratch = torch.empty(nbytes + 256, device=x.device, dtype=torch.uint8)
+        out = torch.empty((T, H), device=x.device, dtype=x.dtype)
+        status = lib.moe_block_fwd(
+            x.data_ptr(), router_logits.data_ptr(), gate_proj.data_ptr(), up_proj.data_ptr(), down_proj.data_ptr(),
+            out.data_ptr(), T, H, I, E, k, int(norm_topk_prob), code, (scratch.data_ptr() + 255) & ~255, nbytes,
+            _lib.stream_ptr(x.device))
+    if status == _lib.ERR_UNSUPPORTED:
+        return None
+    _lib.check(status, "moe_block_fwd")
+    return out
+
+
 def moe_block_forward(hidden_states: torch.Tensor, gate_weight: torch.Tensor, gate_proj: torch.Tensor,
                       up_proj: torch.Tensor, down_proj: torch.Tensor, num_selected: int,
                       norm_topk_prob: bool = True) -> tuple[torch.Tensor, torch.Tensor]:
@@ -72,6 +102,10 @@ def moe_block_forward(hidden_states: torch.Tensor, gate_weight: torch.Tensor, ga
     k = num_selected
     x = hidden_states.reshape(T, H)
     router_logits = torch.nn.functional.linear(x, gate_weight)
+    if not torch.is_grad_enabled() and not GATHER_IN_KERNEL:
+        out = _block_infer(x, router_logits, gate_proj, up_proj, down_proj, k, norm_topk_prob)
+        if out is not None:
+            return out.view(B, S, H), router_logits
     routing_weights, selected = route(router_logits, k, norm_topk_prob, x.dtype)
     m_sizes, sort_idx, inv_sort_idx = get_expert_counts_and_idx(selected.view(T * k), E)
     if not torch.is_grad_enabled() and GATHER_IN_KERNEL:
