@@ -762,10 +762,10 @@ def main():
     comm_stream = torch.cuda.Stream(device=dev) if world > 1 else None
     ev = lambda: torch.cuda.Event(enable_timing=True)
     kernel_ms = {"fwd": [], "dx": [], "dw": []}
-    # three GEMMs, each preceded by the kernel that builds its per-expert tensor maps; per step at
-    # N > 1 also two row pushes (peer) or four row permutations (nccl)
+    # three GEMMs; per step at N > 1 also two row pushes and the kernels that build the output maps of the scattered
+    # forward and dX (peer) or four row permutations (nccl)
     nck = max(1, min(args.ep_chunks, E_local))
-    launches_per_step = 6 if world == 1 else (8 * nck + (2 if peer["dedup"] else 0) if args.ep_transport == "peer" else 10)
+    launches_per_step = 3 if world == 1 else (7 * nck + (2 if peer["dedup"] else 0) if args.ep_transport == "peer" else 7)
 
     def step_resident(record: bool):
         if world == 1:
@@ -1143,7 +1143,7 @@ def main():
                     "note": "inputs double-buffered: the upload of step i+1 runs beside the compute of step i; y, dX, dW and "
                             "m_sizes of every step are copied back into pinned host memory inside the timed region",
                     "tokens_per_s": T * world / (e2e_ms * 1e-3), "clocks": e2e_clocks},
-            "gpu_launches": args.steps * (2 if args.only else launches_per_step),
+            "gpu_launches": args.steps * (1 if args.only else launches_per_step),
             "tokens_per_s": T * world / (resident_ms * 1e-3),
             "clocks": clocks, "kernel_wait_errors": err_flag,
         }

@@ -104,11 +104,11 @@ int moe_batch_begins_ends(const void* s_sorted, int s_dtype, int64_t M, int E,
  * consecutive rows (m_sizes_dtype MOE_I32 or MOE_I64, sum = M, zeros allowed).
  * Accumulation is fp32; the result is rounded once to dtype_out.
  * ws/ws_bytes: device scratch of moe_grouped_gemm_workspace_bytes() bytes, 128-byte aligned,
- *   owned by the caller.  dW, the NF4 and the scattered forms launch a small kernel ahead of the
- *   GEMM that writes per-expert tensor maps and a work-item counter into it, so one workspace serves
- *   one GEMM at a time: calls issued on one stream may share it, calls on different streams need one
- *   each.  Forward and dX accept NULL/0 (they do not use it); dW on the tensor-core path and the
- *   fused / gathered / scattered forms return MOE_ERR_WORKSPACE.
+ *   owned by the caller.  The NF4 and the scattered forms launch a small kernel ahead of the GEMM
+ *   that writes per-expert tensor maps into it, so one workspace serves one GEMM at a time: calls
+ *   issued on one stream may share it, calls on different streams need one each.  The other forms do
+ *   not use it; forward and dX accept NULL/0, dW on the tensor-core path and the fused / gathered
+ *   forms return MOE_ERR_WORKSPACE.
  * ------------------------------------------------------------------------------- */
 size_t moe_grouped_gemm_workspace_bytes(int which /*0 fwd, 1 dx, 2 dw*/, int64_t M, int N, int K, int E);
 

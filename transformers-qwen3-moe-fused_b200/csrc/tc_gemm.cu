@@ -42,7 +42,6 @@ struct GemmParams {
   uint32_t idesc;
   const CUtensorMap* group_maps = nullptr;  // per-expert tensor maps in workspace ([slot][expert]), or null
   const int* weight_index = nullptr;  // weight slice of each group (null: group e uses slice e)
-  int* tile_counter = nullptr;  // work items are drawn from this counter (zeroed by build_group_maps_kernel); null: round-robin
   int stages = 0;               // CTA-pair forward / dX: depth of the operand ring
   int ld_out = 0;               // single-CTA forward / dX: row pitch of the output (0: N)
   float alpha[2] = {1.f, 1.f};  // single-CTA forward / dX: factors of the columns before / from b_split on
@@ -728,14 +727,13 @@ static int launch_pair(void (*kernel)(KArgs...), int grid, int smem_bytes, cudaS
 template <typename... KArgs, typename... Args>
 static int launch_pair_threads(void (*kernel)(KArgs...), int grid, int threads, int smem_bytes, cudaStream_t stream, Args... args);
 
-// Workspace of the tensor-core grouped GEMMs: GroupMapTemplates::MAX per-expert tensor maps per expert
-// (slot-major, 128 bytes each), then the work-item counter of the launch.
+// Workspace of the tensor-core grouped GEMMs: GroupMapTemplates::MAX per-expert tensor maps per expert (slot-major, 128
+// bytes each) for the NF4 and scattered forms, and 128 bytes that are not in use.
 static size_t ws_maps_bytes(int E) { return (size_t)tc::GroupMapTemplates::MAX * (size_t)E * sizeof(CUtensorMap); }
 size_t tc_workspace_bytes(int E) { return E > 0 ? ws_maps_bytes(E) + 128 : 0; }
 static bool ws_usable(const void* ws, size_t ws_bytes, int E) {
   return ws != nullptr && (((uintptr_t)ws & 127) == 0) && ws_bytes >= tc_workspace_bytes(E);
 }
-static int* ws_counter(void* ws, int E) { return reinterpret_cast<int*>(reinterpret_cast<uint8_t*>(ws) + ws_maps_bytes(E)); }
 
 // Shared-memory footprint of the CTA-pair forward / dX kernels with `stages` ring slots.
 static int pair_smem_bytes(int stages, int E) {
@@ -832,7 +830,7 @@ static int pair_grouped_gemm(int which, const PairOperand* ops, int n_ops, const
     tm.t[GM_OUT] = maps.out;
     const int gm_smem = 8 * 128 + 2 * (E + 1) * 4 + 128;
     build_group_maps_kernel<<<(E + 7) / 8, 256, gm_smem, stream>>>(tm, m_sizes, ms64, E, M, reinterpret_cast<CUtensorMap*>(ws),
-                                                                   nullptr, out_ptrs, GM_OUT, (int64_t)N * 2);
+                                                                   out_ptrs, GM_OUT, (int64_t)N * 2);
     if ((st = launch_status()) != MOE_OK) return st;
     p.group_maps = reinterpret_cast<const CUtensorMap*>(ws);
   }
@@ -874,27 +872,17 @@ static int dw_grouped_gemm(const void* x, const void* dy, const void* m_sizes, i
   if (!ws_usable(ws, ws_bytes, E)) return MOE_ERR_WORKSPACE;
   GemmParams p;
   p.m_sizes = m_sizes; p.out = out; p.M = M; p.N = N; p.K = K; p.E = E; p.ms64 = ms64; p.dtype_out = dtype_out;
-  p.group_maps = reinterpret_cast<const CUtensorMap*>(ws);
-  p.tile_counter = ws_counter(ws, E);
   if ((int64_t)E * ((N + 127) / 128) * (int64_t)((K + 127) / 128) >= (int64_t)1 << 30) return MOE_ERR_UNSUPPORTED;  // 32-bit work-item ids
   const int fmt = dtype_in == MOE_BF16 ? 1 : 0;
   int st;
-  GroupMapTemplates tm;
-  tm.mask = (1 << GM_DY) | (1 << GM_X);
-  if ((st = make_map(&tm.t[GM_DY], dtype_in, dy, (uint64_t)N, (uint64_t)M, 0, BK, (uint64_t)ldy)) != MOE_OK) return st;
-  if ((st = make_map(&tm.t[GM_X], dtype_in, x, (uint64_t)K, (uint64_t)M, 0, BK, (uint64_t)ldx)) != MOE_OK) return st;
-  const int gm_smem = 8 * 128 + 2 * (E + 1) * 4 + 128;
-  build_group_maps_kernel<<<(E + 7) / 8, 256, gm_smem, stream>>>(tm, m_sizes, ms64, E, M, reinterpret_cast<CUtensorMap*>(ws),
-                                                                 ws_counter(ws, E));
-  if ((st = launch_status()) != MOE_OK) return st;
-
-  const bool staged = dtype_out != MOE_F32;
-  CUtensorMap mo;
-  if (staged) {
-    if ((st = make_map(&mo, dtype_out, out, (uint64_t)K, (uint64_t)N, (uint64_t)E, 128)) != MOE_OK) return st;
-  } else {
-    memset(&mo, 0, sizeof(mo));
+  DwMaps maps;
+  memset(&maps, 0, sizeof(maps));
+  for (int b = 0; b < DW_BOXES; ++b) {
+    if ((st = make_map(&maps.dy[b], dtype_in, dy, (uint64_t)N, (uint64_t)M, 0, dw_box_rows(b), (uint64_t)ldy)) != MOE_OK) return st;
+    if ((st = make_map(&maps.x[b], dtype_in, x, (uint64_t)K, (uint64_t)M, 0, dw_box_rows(b), (uint64_t)ldx)) != MOE_OK) return st;
   }
+  const bool staged = dtype_out != MOE_F32;
+  if (staged && (st = make_map(&maps.out, dtype_out, out, (uint64_t)K, (uint64_t)N, (uint64_t)E, 128)) != MOE_OK) return st;
   const int tables = 2 * (E + 1) * 4 + (int)sizeof(DwControl) + 1024 + 2 * 128 * 128;
   const bool pair = !single_cta && staged && N >= 192 && K >= 192 && (((uintptr_t)out & 15) == 0);
   if (pair) {
@@ -904,21 +892,22 @@ static int dw_grouped_gemm(const void* x, const void* dy, const void* m_sizes, i
     p.idesc = make_idesc(fmt, 1, 1, 256, 256);
     auto kern = dw_kernel<true, 256, ST>;
     if ((st = set_smem(kern, bytes)) != MOE_OK) return st;
-    return launch_pair(kern, 2 * resident_pairs(kern, bytes), bytes, stream, mo, p);
+    return launch_pair(kern, 2 * E * ((N + 255) / 256) * ((K + 255) / 256), bytes, stream, maps, p);
   }
+  auto items = [&](int bn) { return (unsigned)(E * ((N + 127) / 128) * ((K + bn - 1) / bn)); };  // one CTA per work item
   if (K > 128) {
     p.idesc = make_idesc(fmt, 1, 1, BM, 256);
     const int bytes4 = 4 * 6 * BK * 128 + tables;
     if (bytes4 <= SMEM_LIMIT) {
       auto kern = dw_kernel<false, 256, 4>;
       if ((st = set_smem(kern, bytes4)) != MOE_OK) return st;
-      kern<<<sm_count(), 192, bytes4, stream>>>(mo, p);
+      kern<<<items(256), 192, bytes4, stream>>>(maps, p);
     } else {
       const int bytes3 = 3 * 6 * BK * 128 + tables;
       if (bytes3 > SMEM_LIMIT) return MOE_ERR_UNSUPPORTED;
       auto kern = dw_kernel<false, 256, 3>;
       if ((st = set_smem(kern, bytes3)) != MOE_OK) return st;
-      kern<<<sm_count(), 192, bytes3, stream>>>(mo, p);
+      kern<<<items(256), 192, bytes3, stream>>>(maps, p);
     }
   } else {
     p.idesc = make_idesc(fmt, 1, 1, BM, 128);
@@ -926,7 +915,7 @@ static int dw_grouped_gemm(const void* x, const void* dy, const void* m_sizes, i
     if (bytes > SMEM_LIMIT) return MOE_ERR_UNSUPPORTED;
     auto kern = dw_kernel<false, 128, 6>;
     if ((st = set_smem(kern, bytes)) != MOE_OK) return st;
-    kern<<<sm_count(), 192, bytes, stream>>>(mo, p);
+    kern<<<items(128), 192, bytes, stream>>>(maps, p);
   }
   return launch_status();
 }
@@ -1149,7 +1138,7 @@ int tc_grouped_gemm_nf4(const void* x, const uint8_t* packed, const float* code,
           if ((st = make_map(&tm.t[GM_OUT], dtype_out, out, (uint64_t)N, (uint64_t)M, 0, 32)) != MOE_OK) return st;
         }
         const int gm_smem = 8 * 128 + 2 * (E + 1) * 4 + 128;
-        build_group_maps_kernel<<<(E + 7) / 8, 256, gm_smem, stream>>>(tm, m_sizes, ms64, E, M, reinterpret_cast<CUtensorMap*>(ws), nullptr);
+        build_group_maps_kernel<<<(E + 7) / 8, 256, gm_smem, stream>>>(tm, m_sizes, ms64, E, M, reinterpret_cast<CUtensorMap*>(ws));
         if ((st = launch_status()) != MOE_OK) return st;
         p.group_maps = reinterpret_cast<const CUtensorMap*>(ws);
       }

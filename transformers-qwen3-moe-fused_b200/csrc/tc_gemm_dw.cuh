@@ -1,23 +1,23 @@
 // Weight-gradient grouped GEMM, w[e,n,k] = sum_{t in group e} dy[t,n] * x[t,k], and the
-// set-up kernel that derives per-expert tensor maps.  Included by tc_gemm.cu.
+// set-up kernel that derives per-expert tensor maps for the scattered and NF4 forms.  Included by tc_gemm.cu.
 //
-// Per-expert tensor maps.  The reduction runs over an expert's rows in blocks of 64; the
-// last block reaches past the group's end into the next expert's rows.  Instead of
-// zeroing those rows in shared memory, every expert gets its own copy of the dy / x tensor
-// maps whose row extent ends at the group's last row, so TMA zero-fills the overhang (and
-// does not even fetch it).  The copies are produced on the device from m_sizes by
-// build_group_maps_kernel (tensormap.replace + tensormap.cp_fenceproxy) into caller-provided
-// workspace, one launch before the GEMM.
+// The reduction runs over an expert's rows in blocks of 64.  The last block of an expert holds rem <= 64 rows, and what
+// follows them in memory belongs to the next expert: its MMA steps of 16 rows must find zeros there (in both operands,
+// an infinity times zero would not do).  TMA brings whole groups of 16 rows in one box, and the last, partial group as
+// boxes of 8, 4, 2 and 1 rows that end exactly at the expert's last row; the rest of the group is filled by boxes that
+// start past the tensor's last row, which TMA fills with zeros.  At most five boxes per operand chunk and expert, on maps
+// that do not depend on the groups.  (Per-expert maps whose row extent ends at the group did the same before: a launch of
+// its own in front of each GEMM, 5.5 us and a gap, with the same time in the GEMM.  Forward + dX + dW: 294 -> 286 us at
+// 5003 rows 2048 -> 768, 1036 -> 1021 us at 65536 rows 2048 -> 1536.)
 //
 // dw_kernel<PAIR, BN>
 //   PAIR = false: one CTA per work item (expert, 128 weight rows, BN weight columns)
 //   PAIR = true : a CTA pair per work item (expert, 256 weight rows, 256 weight columns),
 //                 tcgen05 cta_group::2; both CTAs' loads complete on the leader's barrier
-// Work items are ordered by decreasing group size and handed out one by one from a global
-// counter (drawn by the otherwise idle warp 1 of the non-leader CTA and passed to the working
-// roles through a ring in shared memory): longest items first onto whichever CTA pair is free,
-// so one expert with a quarter of the rows does not leave most of the GPU waiting for the few
-// pairs that drew its items.  Without a counter the items are dealt round-robin.
+// Work items are ordered by decreasing group size, one cluster (CTA) of the grid each; a running pair takes over the next
+// one that has not started (cluster launch control, as in the forward): longest items first onto whichever pair is
+// free, so one expert with a quarter of the rows does not leave most of the GPU waiting for the few pairs that drew
+// its items.
 // The last reduction block of an expert only issues the MMA k-steps that hold real rows.
 // 16-bit outputs leave through a swizzled staging tile and TMA stores (the output has no ragged
 // dimension; TMA clips at N and K); fp32 outputs (single-CTA form only) are stored from registers.
@@ -34,22 +34,19 @@ struct GroupMapTemplates {
 
 // out[t * E + e] = templates.t[t] with the extent of dimension 1 (rows) set to the last row
 // of expert e (exclusive), for every slot t of templates.mask.  One warp per expert.
-// Also resets the work-item counter of the GEMM launched after it.
 // With `out_ptrs`, slot `ptr_slot` of group e is additionally re-based so that row row_start[e]
 // of the map is the address out_ptrs[e]: each group's rows then land in a buffer of their own
 // (possibly in a peer GPU's memory) while the kernels keep addressing rows by their position in
 // the concatenated input.  `row_bytes` is the pitch of that slot's rows.
 __global__ void __launch_bounds__(256)
 build_group_maps_kernel(const __grid_constant__ GroupMapTemplates tm, const void* __restrict__ m_sizes, int ms64,
-                        int E, int64_t M, CUtensorMap* __restrict__ out, int* __restrict__ counters,
+                        int E, int64_t M, CUtensorMap* __restrict__ out,
                         const uint64_t* __restrict__ out_ptrs = nullptr, int ptr_slot = -1, int64_t row_bytes = 0) {
   extern __shared__ uint8_t gm_smem_raw[];
   uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(gm_smem_raw) + 127) & ~(uintptr_t)127);
   CUtensorMap* slots = reinterpret_cast<CUtensorMap*>(base);  // 8 slots, one per warp
   int* row_start = reinterpret_cast<int*>(base + 8 * 128);
   int* scratch = row_start + (E + 1);
-  // the GEMM that follows draws its work items from counters[0]
-  if (counters != nullptr && blockIdx.x == 0 && threadIdx.x == 0) counters[0] = 0;
   build_group_tables(m_sizes, ms64, E, M, 64, row_start, scratch);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int e = blockIdx.x * 8 + warp;
@@ -76,7 +73,14 @@ build_group_maps_kernel(const __grid_constant__ GroupMapTemplates tm, const void
   }
 }
 
-enum { GM_DY = 0, GM_X = 1 };  // slots of the dW kernel's per-expert maps
+// Maps of dy and x with boxes of 64 columns and DW_BOX rows.
+constexpr int DW_BOXES = 6;
+__host__ __device__ constexpr int dw_box_rows(int b) { return b == 0 ? 64 : b == 1 ? 16 : 16 >> (b - 1); }  // 64, 16, 8, 4, 2, 1
+struct DwMaps {
+  CUtensorMap dy[DW_BOXES];
+  CUtensorMap x[DW_BOXES];
+  CUtensorMap out;
+};
 
 struct DwControl {
   uint64_t full[8];
@@ -84,13 +88,15 @@ struct DwControl {
   uint64_t tmem_full[2];
   uint64_t tmem_empty[2];
   SchedRing sched;
+  uint64_t cancel_bar;
+  alignas(16) uint4 cancel_response;
   uint32_t tmem_base;
   int abort_flag;
 };
 
 template <bool PAIR, int BN, int STAGES>
 __global__ void __launch_bounds__(192, 1)
-dw_kernel(const __grid_constant__ CUtensorMap tmap_out, const GemmParams p) {
+dw_kernel(const __grid_constant__ DwMaps maps, const GemmParams p) {
   constexpr int ROWS = PAIR ? 256 : 128;          // weight rows per work item
   constexpr int B_CHUNKS = PAIR ? 2 : BN / 64;    // 64-wide chunks of the x operand staged per CTA
   constexpr int CHUNK_BYTES = BK * 128;           // 64 reduction rows x 128 B
@@ -116,9 +122,12 @@ dw_kernel(const __grid_constant__ CUtensorMap tmap_out, const GemmParams p) {
     for (int s = 0; s < STAGES; ++s) { mbar_init(&ctl->full[s], 1); mbar_init(&ctl->empty[s], 1); }
     for (int a = 0; a < 2; ++a) { mbar_init(&ctl->tmem_full[a], 1); mbar_init(&ctl->tmem_empty[a], 4 * NCTA); }
     TileFeed<NCTA>::init(&ctl->sched);
+    mbar_init(&ctl->cancel_bar, 1);
     ctl->abort_flag = 0;
     fence_barrier_init();
-    tma_prefetch_desc(&tmap_out);
+    tma_prefetch_desc(&maps.out);
+    tma_prefetch_desc(&maps.dy[0]);
+    tma_prefetch_desc(&maps.x[0]);
   }
   if (warp == 1) {
     if constexpr (PAIR) { tmem_alloc_pair(&ctl->tmem_base, TMEM_COLS); tmem_relinquish_pair(); }
@@ -153,8 +162,6 @@ dw_kernel(const __grid_constant__ CUtensorMap tmap_out, const GemmParams p) {
   const int k_tiles = (p.K + BN - 1) / BN;
   const int per_expert = n_tiles * k_tiles;
   const int total_items = p.E * per_expert;
-  const int G = PAIR ? (gridDim.x >> 1) : gridDim.x;
-  const int unit = PAIR ? (blockIdx.x >> 1) : blockIdx.x;
   if (warp == 0) {
     // ------------------------------ TMA producer ------------------------------
     if (elect_one()) {
@@ -162,25 +169,21 @@ dw_kernel(const __grid_constant__ CUtensorMap tmap_out, const GemmParams p) {
       const uint32_t full0 = PAIR ? map_to_cta(smem_u32(&ctl->full[0]), 0) : smem_u32(&ctl->full[0]);
       uint32_t it = 0;
       bool ok = true;
-      int last_e = -1;
-      // single-CTA form: this thread also draws the work items (the value of a draw is first looked
-      // at one item later, so that the atomic's round trip overlaps the loads in between)
-      uint32_t drawn = 0;
-      auto draw = [&]() -> int64_t {
-        const int64_t t = drawn == 0 ? (int64_t)unit : p.tile_counter ? (int64_t)atomicAdd(p.tile_counter, 1) + G
-                                                                      : (int64_t)unit + (int64_t)drawn * G;
-        ++drawn;
-        return t;
-      };
-      int64_t next = PAIR ? 0 : draw();
+      // single-CTA form: this thread also draws the work items (it asks for the next one before the loads of an item
+      // and looks at the answer after them)
+      int next = (int)blockIdx.x;
+      uint32_t draw_ph = 0;
       while (ok) {
         int item;
         if constexpr (PAIR) {
           item = feed.take();
         } else {
-          item = next < total_items ? (int)next : -1;
+          item = next;
           if (!feed.publish(item)) break;
-          if (item >= 0) next = draw();
+          if (item >= 0) {
+            mbar_expect_tx(&ctl->cancel_bar, 16);
+            cluster_try_cancel(&ctl->cancel_response, &ctl->cancel_bar);
+          }
         }
         if (item < 0) break;
         const int e = sorted[item / per_expert];
@@ -189,9 +192,6 @@ dw_kernel(const __grid_constant__ CUtensorMap tmap_out, const GemmParams p) {
         const int k0 = (j / n_tiles) * BN + (PAIR ? (int)rank * 128 : 0);
         const int r0 = row_start[e];
         const int m_blocks = (row_start[e + 1] - r0 + BK - 1) / BK;
-        const CUtensorMap* mdy = p.group_maps + (size_t)GM_DY * p.E + e;
-        const CUtensorMap* mx = p.group_maps + (size_t)GM_X * p.E + e;
-        if (e != last_e && m_blocks > 0) { tensormap_acquire(mdy); tensormap_acquire(mx); last_e = e; }
         for (int mb = 0; mb < m_blocks; ++mb, ++it) {
           const int s = it % STAGES;
           const uint32_t ph = (it / STAGES) & 1;
@@ -199,19 +199,48 @@ dw_kernel(const __grid_constant__ CUtensorMap tmap_out, const GemmParams p) {
           uint8_t* sa = smem + s * STAGE_BYTES;
           uint8_t* sb = sa + 2 * CHUNK_BYTES;
           const uint32_t bar = full0 + s * 8;
-          if (leader) mbar_expect_tx(&ctl->full[s], NCTA * STAGE_BYTES);
           const int row = r0 + mb * BK;
-          if constexpr (PAIR) {
-            tma_load_2d_pair(sa, mdy, bar, n0, row);
-            tma_load_2d_pair(sa + CHUNK_BYTES, mdy, bar, n0 + 64, row);
+          const int left = row_start[e + 1] - row;  // rows of this block
+          auto load = [&](const CUtensorMap* map, uint8_t* dst, int x, int y) {
+            if constexpr (PAIR) tma_load_2d_pair(dst, map, bar, x, y);
+            else tma_load_2d(dst, map, &ctl->full[s], x, y);
+          };
+          // rows [at, at + box rows) of all chunks of the stage, from tensor row y on
+          auto load_rows = [&](int box, int at, int y) {
+            load(&maps.dy[box], sa + at * 128, n0, y);
+            load(&maps.dy[box], sa + CHUNK_BYTES + at * 128, n0 + 64, y);
 #pragma unroll
-            for (int c = 0; c < B_CHUNKS; ++c) tma_load_2d_pair(sb + c * CHUNK_BYTES, mx, bar, k0 + c * 64, row);
+            for (int c = 0; c < B_CHUNKS; ++c) load(&maps.x[box], sb + c * CHUNK_BYTES + at * 128, k0 + c * 64, y);
+          };
+          if (left >= BK) {
+            if (leader) mbar_expect_tx(&ctl->full[s], NCTA * STAGE_BYTES);
+            load_rows(0, 0, row);
           } else {
-            tma_load_2d(sa, mdy, &ctl->full[s], n0, row);
-            tma_load_2d(sa + CHUNK_BYTES, mdy, &ctl->full[s], n0 + 64, row);
-#pragma unroll
-            for (int c = 0; c < B_CHUNKS; ++c) tma_load_2d(sb + c * CHUNK_BYTES, mx, &ctl->full[s], k0 + c * 64, row);
+            const int steps = (left + 15) >> 4, tail = left & 15;
+            if (leader) mbar_expect_tx(&ctl->full[s], NCTA * (uint32_t)(steps * 16 * 128 * (2 + B_CHUNKS)));
+            for (int g = 0; g < (left >> 4); ++g) load_rows(1, g * 16, row + g * 16);
+            if (tail) {
+              // halve the group down to the boundary: real rows before it, rows past the tensor (zeros) behind it
+              const int base = left & ~15;
+              int lo = 0, hi = 16;  // the boundary lies in (lo, hi]
+              for (int box = 2; box < DW_BOXES && tail > lo && tail < hi; ++box) {
+                const int mid = lo + dw_box_rows(box);
+                if (tail >= mid) { load_rows(box, base + lo, row + base + lo); lo = mid; }
+                else { load_rows(box, base + mid, (int)p.M); hi = mid; }
+              }
+              // [lo, hi) is all real (tail == hi) or all behind the boundary (tail == lo); its size is a box's
+              const int rest = hi - lo;
+              const int box = rest == 8 ? 2 : rest == 4 ? 3 : rest == 2 ? 4 : 5;
+              if (rest > 0) load_rows(box, base + lo, tail == hi ? row + base + lo : (int)p.M);
+            }
           }
+        }
+        if constexpr (!PAIR) {
+          if (!ok) break;
+          if (!mbar_wait(&ctl->cancel_bar, draw_ph, abort_flag, PW_CANCEL)) break;
+          draw_ph ^= 1;
+          next = cluster_cancelled_cta(&ctl->cancel_response);
+          fence_proxy_async_smem();  // the response has been read before the next one may be written
         }
       }
     }
@@ -221,7 +250,7 @@ dw_kernel(const __grid_constant__ CUtensorMap tmap_out, const GemmParams p) {
       // (CTA pairs only) this warp has no MMAs to issue in the non-leader CTA: it draws the work items
       if (elect_one()) {
         TileFeed<NCTA> feed(&ctl->sched, abort_flag);
-        feed.run(p.tile_counter, total_items, unit, G);
+        feed.run_cancel(&ctl->cancel_bar, &ctl->cancel_response, total_items, (int)(blockIdx.x >> 1));
       }
     } else if (elect_one()) {
       TileFeed<NCTA> feed(&ctl->sched, abort_flag);
@@ -352,7 +381,7 @@ dw_kernel(const __grid_constant__ CUtensorMap tmap_out, const GemmParams p) {
         fence_proxy_async_smem();
         named_barrier_sync(1, 128);
         if (epi_tid == 0) {
-          tma_store_3d(&tmap_out, buf, k0 + c * 64, n0, e);  // rows / columns past N / K are clipped
+          tma_store_3d(&maps.out, buf, k0 + c * 64, n0, e);  // rows / columns past N / K are clipped
           tma_store_commit();
         }
       }

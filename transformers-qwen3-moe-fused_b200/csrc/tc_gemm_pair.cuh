@@ -236,8 +236,8 @@ __device__ __forceinline__ void pair_store_tile_gate_up(uint8_t* staging, uint32
 // in the drawing thread's CTA; one arrival per reader) says everybody has read it.
 //   NCTA = 2: the drawing thread is a thread of its own (warp 1 of the non-leader CTA, which has no
 //             MMAs to issue); readers: both producers, the MMA thread, 8 epilogue warps.  It runs up
-//             to SCHED_DEPTH tiles ahead, so the round trip of its atomicAdd is never waited for.
-//   NCTA = 1: the producer thread draws for itself; readers: the MMA thread, 4 epilogue warps.
+//             to SCHED_DEPTH tiles ahead, so the round trip of its request is never waited for.
+//   NCTA = 1: the producer thread draws for itself (dW); readers: the MMA thread, 4 epilogue warps.
 template <int NCTA>
 struct TileFeed {
   static constexpr int READERS = NCTA == 2 ? 11 : 5;
@@ -279,18 +279,8 @@ struct TileFeed {
     ++n;
     return true;
   }
-  // Body of the drawing thread when it has nothing else to do (NCTA = 2).  The first tile of pair `first`
-  // is tile `first`; further ids come from the global counter (offset by the `stride` pairs), or
-  // round-robin without one.  (When the first ids were drawn too, the pairs that started a little earlier
-  // took several tiles each before the others had one.)
-  __device__ __forceinline__ void run(int* counter, int total, int first, int stride) {
-    for (int64_t t = first;; t = counter ? (int64_t)atomicAdd(counter, 1) + stride : t + stride) {
-      const int tile = t < total ? (int)t : -1;
-      if (!publish(tile) || tile < 0) return;
-    }
-  }
-  // The same with the tiles of the clusters that have not started yet: `first` is this cluster's own tile;
-  // ids from `total` on (the grid is an upper bound) are passed over.
+  // Body of the drawing thread when it has nothing else to do (NCTA = 2): the tiles of the clusters that have not
+  // started yet, after this cluster's own tile `first`; ids from `total` on (the grid is an upper bound) are passed over.
   __device__ __forceinline__ void run_cancel(uint64_t* bar, uint4* response, int total, int first) {
     uint32_t ph = 0;
     for (int tile = first;;) {
