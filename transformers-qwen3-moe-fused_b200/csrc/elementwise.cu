@@ -440,8 +440,9 @@ combine_kernel(const T* __restrict__ y, const int32_t* __restrict__ inv_sort_idx
 //   dy[r, :] = T(f32(weights[s]) * f32(dout[t, :]))      dweights[s] = T(sum_c f32(dout[t, c]) * f32(y[r, c]))
 // in one pass over y and dy.  Bound by HBM: y is read and dy written once; the k slots of a token are
 // neighbouring warps, so its dout row comes from L1 / L2 after the first.  A warp per slot (not a CTA per
-// token) keeps the reduction in shuffles and every lane at eight 16-byte loads of y in flight.  Measured at
-// 8191 tokens x 8, H = 2048, bf16: 120 us (4.8 TB/s); the gathers, products and reduction in ATen took 1000 us.
+// token) keeps the reduction in shuffles; a lane has four 16-byte loads of y and four of dout in flight (with eight of
+// y first and each of dout where it was used, the dout loads waited one after the other: 120 us).  Measured at
+// 8191 tokens x 8, H = 2048, bf16: 91 us (6.3 TB/s); the gathers, products and reduction in ATen took 1000 us.
 template <typename T, bool VEC, bool WANT_DY, bool WANT_DW>
 __global__ void __launch_bounds__(EW_THREADS)
 combine_bwd_kernel(const T* __restrict__ dout, const T* __restrict__ y, const int32_t* __restrict__ inv_sort_idx,
@@ -454,30 +455,29 @@ combine_bwd_kernel(const T* __restrict__ dout, const T* __restrict__ y, const in
     const float w = WANT_DY ? to_f32(weights[s]) : 0.f;
     float dot = 0.f;
     if constexpr (VEC) {
-      constexpr int V = Vec<T>::N, UNROLL = 8;
+      constexpr int V = Vec<T>::N, UNROLL = 4;
       const int row_vecs = H / V;
       for (int c0 = 0; c0 < row_vecs; c0 += 32 * UNROLL) {
-        Vec<T> vy[UNROLL];
-        if constexpr (WANT_DW) {
+        Vec<T> vy[UNROLL], vdo[UNROLL];
 #pragma unroll
-          for (int u = 0; u < UNROLL; ++u) {
-            const int c = c0 + u * 32 + lane;
-            if (c < row_vecs) *reinterpret_cast<uint4*>(vy[u].v) = __ldcs(reinterpret_cast<const uint4*>(y + r * H) + c);
-          }
+        for (int u = 0; u < UNROLL; ++u) {
+          const int c = c0 + u * 32 + lane;
+          if (c >= row_vecs) continue;
+          if constexpr (WANT_DW) *reinterpret_cast<uint4*>(vy[u].v) = __ldcs(reinterpret_cast<const uint4*>(y + r * H) + c);
+          vdo[u] = load_vec(src + c * V);
         }
 #pragma unroll
         for (int u = 0; u < UNROLL; ++u) {
           const int c = c0 + u * 32 + lane;
           if (c >= row_vecs) continue;
-          const Vec<T> vd = load_vec(src + c * V);
           Vec<T> o;
 #pragma unroll
           for (int i = 0; i < V; ++i) {
-            const float d = to_f32(vd.v[i]);
+            const float d = to_f32(vdo[u].v[i]);
             if constexpr (WANT_DY) o.v[i] = from_f32<T>(w * d);
             if constexpr (WANT_DW) dot = fmaf(d, to_f32(vy[u].v[i]), dot);
           }
-          if constexpr (WANT_DY) store_vec(dy + r * H + c * V, o);
+          if constexpr (WANT_DY) __stcs(reinterpret_cast<uint4*>(dy + r * H) + c, *reinterpret_cast<const uint4*>(o.v));
         }
       }
     } else {
