@@ -303,9 +303,12 @@ int moe_lora_project(int which, const void* x, const void* a0, int n0, float s0,
                      const void* m_sizes, int msd, void* y, int64_t ldy, int64_t M, int K, int E, int dtype, void* stream);
 
 /* moe_grouped_gemm_dw on operands whose rows are ldx / ldy elements apart (multiples of 8; dtype in = dtype out).
+ * With w2 the N <= 128 columns of dy belong to two weights that share x: columns before n1 (a multiple of 8) give
+ * w (E, n1, K), the others w2 (E, N - n1, K); both 16-byte aligned.
  * Replaces qwen3_moe_fused/kernels/fast_lora.py:139-149 together with moe_lora_project. */
 int moe_grouped_gemm_dw_strided(const void* x, int64_t ldx, const void* dy, int64_t ldy, const void* m_sizes, int msd,
-                                void* w, int64_t M, int N, int K, int E, int dtype, void* ws, size_t ws_bytes, void* stream);
+                                void* w, void* w2, int n1, int64_t M, int N, int K, int E, int dtype, void* ws,
+                                size_t ws_bytes, void* stream);
 
 /* ---------------------------------------------------------------------------------
  * Expert parallelism over peer memory.  The reference has no multi-GPU path

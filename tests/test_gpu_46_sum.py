@@ -64,6 +64,9 @@ def test_projections_and_strided_dw(cuda, K, n0, n1):
     lora_project(x, a0.transpose(1, 2).contiguous(), 1.75, m_sizes, back[:, :n0], transposed=True)
     dw = grouped_gemm_dw_strided(x, out[:, :n0], m_sizes)
     dwt = grouped_gemm_dw_strided(out[:, :n0], x, m_sizes)
+    both = None
+    if 0 < n1 and n0 + n1 <= 128:  # two weights that share x
+        both = torch.cat(grouped_gemm_dw_strided(x, out[:, :n0 + n1], m_sizes, n1=n0), 1)
     for e, r in groups(SIZES):
         xd = x[r].double()
         for cols, a, s in ((slice(0, n0), a0, 1.75), (slice(n0, n0 + n1), a1, -0.375)):
@@ -75,6 +78,9 @@ def test_projections_and_strided_dw(cuda, K, n0, n1):
                 check(back[r, :n0], ref, mag, K + 2, dtype)
         t = out[r, :n0].double()
         check(dw[e], t.T @ xd, t.abs().T @ xd.abs(), r.stop - r.start + 2, dtype)
+        if both is not None:
+            tb = out[r, :n0 + n1].double()
+            check(both[e], tb.T @ xd, tb.abs().T @ xd.abs(), r.stop - r.start + 2, dtype)
         check(dwt[e], xd.T @ t, xd.abs().T @ t.abs(), r.stop - r.start + 2, dtype)
     assert (out[:, n0 + n1:] == 7.0).all() and (back[:, n0:] == 7.0).all()
 

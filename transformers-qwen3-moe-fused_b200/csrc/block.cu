@@ -115,7 +115,7 @@ MOE_API int moe_lora_mlp_bwd(const moe_lora_weights* w, const moe_lora_grads* gr
   const uint8_t* t_u = (const uint8_t*)t_gu + off;
   uint8_t* d_u = (uint8_t*)d_gu + off;
   auto dw = [&](const void* x_, int64_t ldx, int K, const void* dy_, int64_t ldy, int N, void* out) {
-    return moe_grouped_gemm_dw_strided(x_, ldx, dy_, ldy, m_sizes, msd, out, M, N, K, E, dtype, ws, ws_bytes, stream);
+    return moe_grouped_gemm_dw_strided(x_, ldx, dy_, ldy, m_sizes, msd, out, nullptr, 0, M, N, K, E, dtype, ws, ws_bytes, stream);
   };
   int st;
   if ((st = moe_lora_project(1, dy, w->b[2], rw, w->scale[2], nullptr, 0, 1.f, m_sizes, msd, d_w, rw, M, H, E, dtype, stream)) != MOE_OK) return st;
@@ -132,8 +132,13 @@ MOE_API int moe_lora_mlp_bwd(const moe_lora_weights* w, const moe_lora_grads* gr
   if ((st = dw(t_w, rw, rw, dy, H, H, grads->db[2])) != MOE_OK) return st;
   if ((st = moe_lora_project(1, e, w->b[0], rg, w->scale[0], nullptr, 0, 1.f, m_sizes, msd, d_gu, ld, M, I, E, dtype, stream)) != MOE_OK) return st;
   if ((st = moe_lora_project(1, g, w->b[1], ru, w->scale[1], nullptr, 0, 1.f, m_sizes, msd, d_u, ld, M, I, E, dtype, stream)) != MOE_OK) return st;
-  if ((st = dw(x, H, H, d_gu, ld, rg, grads->da[0])) != MOE_OK) return st;
-  if ((st = dw(x, H, H, d_u, ld, ru, grads->da[1])) != MOE_OK) return st;
+  if (rg + ru <= 128) {  // both gradients of a from one read of x
+    if ((st = moe_grouped_gemm_dw_strided(x, H, d_gu, ld, m_sizes, msd, grads->da[0], grads->da[1], rg, M, rg + ru, H, E, dtype, ws,
+                                          ws_bytes, stream)) != MOE_OK) return st;
+  } else {
+    if ((st = dw(x, H, H, d_gu, ld, rg, grads->da[0])) != MOE_OK) return st;
+    if ((st = dw(x, H, H, d_u, ld, ru, grads->da[1])) != MOE_OK) return st;
+  }
   if ((st = dw(t_gu, ld, rg, e, I, I, grads->db[0])) != MOE_OK) return st;
   if ((st = dw(t_u, ld, ru, g, I, I, grads->db[1])) != MOE_OK) return st;
   if (!dx) return MOE_OK;

@@ -36,8 +36,8 @@ int tc_lora_project(int which, const void* x, const void* a0, int n0, float s0, 
                     const void* m_sizes, int ms64, void* out, int ld_out, int64_t M, int K, int E, int dtype,
                     cudaStream_t stream);
 int tc_grouped_gemm_dw_strided(const void* x, int64_t ldx, const void* dy, int64_t ldy, const void* m_sizes, int ms64,
-                               void* out, int64_t M, int N, int K, int E, int dtype, void* ws, size_t ws_bytes,
-                               cudaStream_t stream);
+                               void* out, void* out2, int n1, int64_t M, int N, int K, int E, int dtype, void* ws,
+                               size_t ws_bytes, cudaStream_t stream);
 int tc_read_error(int* flag_out, bool clear);
 size_t tc_workspace_bytes(int E);
 int tc_read_late_values(int* out);
@@ -267,18 +267,25 @@ MOE_API int moe_lora_project(int which, const void* x, const void* a0, int n0, f
 }
 
 MOE_API int moe_grouped_gemm_dw_strided(const void* x, int64_t ldx, const void* dy, int64_t ldy, const void* m_sizes,
-                                        int msd, void* w, int64_t M, int N, int K, int E, int dtype, void* ws,
-                                        size_t ws_bytes, void* stream) {
+                                        int msd, void* w, void* w2, int n1, int64_t M, int N, int K, int E, int dtype,
+                                        void* ws, size_t ws_bytes, void* stream) {
   if (!is_float_dtype(dtype) || !is_int_dtype(msd)) return MOE_ERR_DTYPE;
   if (M < 0 || N < 0 || K < 0 || E <= 0 || M > 0x7fffffffLL || ldx < K || ldy < N) return MOE_ERR_SHAPE;
   if (!m_sizes) return MOE_ERR_NULL;
   if (N == 0 || K == 0) return MOE_OK;
   if (!w || (M > 0 && (!x || !dy))) return MOE_ERR_NULL;
-  if (M == 0) return cuda_status(cudaMemsetAsync(w, 0, (size_t)E * N * K * dtype_size(dtype), (cudaStream_t)stream));
+  if (w2 && (n1 <= 0 || n1 >= N)) return MOE_ERR_SHAPE;
+  if (M == 0) {
+    const size_t row = (size_t)E * K * dtype_size(dtype);
+    cudaError_t err = cudaMemsetAsync(w, 0, row * (w2 ? n1 : N), (cudaStream_t)stream);
+    if (err == cudaSuccess && w2) err = cudaMemsetAsync(w2, 0, row * (N - n1), (cudaStream_t)stream);
+    return cuda_status(err);
+  }
   if (!device_is_sm100()) return MOE_ERR_DEVICE;
   const int path = g_path.load(std::memory_order_relaxed);
+  if (w2 && (N > 128 || n1 % 8 || (((uintptr_t)w | (uintptr_t)w2) & 15))) return MOE_ERR_UNSUPPORTED;
   if (path == MOE_PATH_SIMT || ldx % 8 || ldy % 8 || !tc_eligible(2, x, dy, w, M, N, K, E, dtype, dtype)) return MOE_ERR_UNSUPPORTED;
-  return tc_grouped_gemm_dw_strided(x, ldx, dy, ldy, m_sizes, msd == MOE_I64, w, M, N, K, E, dtype, ws, ws_bytes,
+  return tc_grouped_gemm_dw_strided(x, ldx, dy, ldy, m_sizes, msd == MOE_I64, w, w2, n1, M, N, K, E, dtype, ws, ws_bytes,
                                     (cudaStream_t)stream);
 }
 

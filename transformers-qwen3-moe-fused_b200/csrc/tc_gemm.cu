@@ -47,6 +47,7 @@ struct GemmParams {
   float alpha[2] = {1.f, 1.f};  // single-CTA forward / dX: factors of the columns before / from b_split on
   int scaled = 0;               //   (applied to the fp32 accumulator, when set)
   int b_split = 0;              // single-CTA forward: columns taken from the first weight (0: there is one weight)
+  int row_split = 0;            // single-CTA dW: rows from here on go to the second output (0: there is one output)
   int staged = 0;               // CTA-pair forward / dX: 16-bit output that may leave by TMA
   const int* row_index = nullptr;  // gathered forms: sorted row r reads row row_index[r] / index_div of the token tensor
   int index_div = 1;
@@ -54,8 +55,8 @@ struct GemmParams {
 };
 
 struct Control {
-  uint64_t full[8];
-  uint64_t empty[8];
+  uint64_t full[12];
+  uint64_t empty[12];
   uint64_t tmem_full[2];
   uint64_t tmem_empty[2];
   uint32_t tmem_base;
@@ -192,14 +193,26 @@ __device__ __forceinline__ void store_acc(void* out, int dtype_out, int64_t dst_
 // ---------------------------------------------------------------------------------------
 // Forward / dX
 // ---------------------------------------------------------------------------------------
+// Stage of the operand ring: 128 activation rows and the weight tile.  Thin outputs (LoRA ranks) are bound by the stream of
+// activation rows, and a CTA keeps no more in flight than its ring holds: as many stages as shared memory takes.
+// (Measured at 32768 rows x 2048, two ranks of 16: 35.4 us with six stages, 33.9 with ten.)
+template <int BN, bool B_MN>
+struct SingleStage {
+  static constexpr int B_CHUNKS = (BN + 63) / 64;  // 64-wide chunks of an MN-major B tile
+  static constexpr int B_BYTES = B_MN ? B_CHUNKS * BK * 128 : (BN < 8 ? 8 : BN) * BK * 2;
+  static constexpr int BYTES = A_STAGE_BYTES + ((B_BYTES + 1023) & ~1023);
+  static constexpr int COUNT = BN == 256 ? 4 : BN == 128 ? 6 : (BYTES > 20480 ? 8 : 10);
+};
+
 template <int BN, bool B_MN>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
 tc_fwd_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
               const GemmParams p, const __grid_constant__ CUtensorMap tmap_b2) {
-  constexpr int B_CHUNKS = (BN + 63) / 64;  // 64-wide chunks of an MN-major B tile
-  constexpr int B_STAGE_BYTES = B_MN ? B_CHUNKS * BK * 128 : (BN < 8 ? 8 : BN) * BK * 2;
-  constexpr int STAGE_BYTES = A_STAGE_BYTES + ((B_STAGE_BYTES + 1023) & ~1023);
-  constexpr int STAGES = (BN == 256) ? 4 : 6;
+  using Stage = SingleStage<BN, B_MN>;
+  constexpr int B_CHUNKS = Stage::B_CHUNKS;
+  constexpr int B_STAGE_BYTES = Stage::B_BYTES;
+  constexpr int STAGE_BYTES = Stage::BYTES;
+  constexpr int STAGES = Stage::COUNT;
   constexpr int ACC_STRIDE = BN < 32 ? 32 : BN;  // TMEM columns between the two accumulators
   constexpr uint32_t TMEM_COLS = 2 * ACC_STRIDE;
 
@@ -617,10 +630,9 @@ static int make_map(CUtensorMap* map, int dtype, const void* base, uint64_t d0, 
   return r == CUDA_SUCCESS ? MOE_OK : MOE_ERR_UNSUPPORTED;
 }
 
-template <int BN>
+template <int BN, bool B_MN>
 static constexpr int smem_bytes_for(int E, int tables) {
-  // upper bound that covers both the K-major and the MN-major B stage of tc_fwd_kernel<BN, *>
-  return ((BN == 256) ? 4 : 6) * (A_STAGE_BYTES + (BN < 64 ? 64 : BN) * BK * 2) + (int)sizeof(Control) + tables * (E + 1) * 4 + 1024;
+  return SingleStage<BN, B_MN>::COUNT * SingleStage<BN, B_MN>::BYTES + (int)sizeof(Control) + tables * (E + 1) * 4 + 1024;
 }
 
 // Per-kernel, per-device memo of launch set-up that does not change between calls: a call of a thin
@@ -867,7 +879,7 @@ static int launch_pair_threads(void (*kernel)(KArgs...), int grid, int threads, 
 // dW on tensor cores: per-expert maps are built into `ws`, then one GEMM launch.
 static int dw_grouped_gemm(const void* x, const void* dy, const void* m_sizes, int ms64, void* out, int64_t M, int N,
                            int K, int E, int dtype_in, int dtype_out, void* ws, size_t ws_bytes, cudaStream_t stream,
-                           bool single_cta, int64_t ldx = 0, int64_t ldy = 0) {
+                           bool single_cta, int64_t ldx = 0, int64_t ldy = 0, void* out2 = nullptr, int n1 = 0) {
   using namespace tc;
   if (!ws_usable(ws, ws_bytes, E)) return MOE_ERR_WORKSPACE;
   GemmParams p;
@@ -882,7 +894,10 @@ static int dw_grouped_gemm(const void* x, const void* dy, const void* m_sizes, i
     if ((st = make_map(&maps.x[b], dtype_in, x, (uint64_t)K, (uint64_t)M, 0, dw_box_rows(b), (uint64_t)ldx)) != MOE_OK) return st;
   }
   const bool staged = dtype_out != MOE_F32;
-  if (staged && (st = make_map(&maps.out, dtype_out, out, (uint64_t)K, (uint64_t)N, (uint64_t)E, 128)) != MOE_OK) return st;
+  if (out2 != nullptr && (!staged || N > 128 || n1 <= 0 || n1 >= N || n1 % 8)) return MOE_ERR_UNSUPPORTED;
+  p.row_split = out2 != nullptr ? n1 : 0;
+  if (staged && (st = make_map(&maps.out, dtype_out, out, (uint64_t)K, (uint64_t)(out2 ? n1 : N), (uint64_t)E, 128)) != MOE_OK) return st;
+  if (out2 && (st = make_map(&maps.out2, dtype_out, out2, (uint64_t)K, (uint64_t)(N - n1), (uint64_t)E, (uint32_t)(128 - n1))) != MOE_OK) return st;
   const int tables = 2 * (E + 1) * 4 + (int)sizeof(DwControl) + 1024 + 2 * 128 * 128;
   const bool pair = !single_cta && staged && N >= 192 && K >= 192 && (((uintptr_t)out & 15) == 0);
   if (pair) {
@@ -957,7 +972,7 @@ static int single_grouped_gemm(int which, const void* a, const void* b, const vo
   p.idesc = make_idesc(fmt, 0, which == 1, BM, bn);
 #define MOE_TC_LAUNCH(BN_, BMN_)                                                              \
   do {                                                                                        \
-    const int bytes = smem_bytes_for<BN_>(E, 2);                                              \
+    const int bytes = smem_bytes_for<BN_, BMN_>(E, 2);                                              \
     if (bytes > SMEM_LIMIT) return MOE_ERR_UNSUPPORTED;                                       \
     if ((st = set_smem(tc_fwd_kernel<BN_, BMN_>, bytes)) != MOE_OK) return st;                \
     tc_fwd_kernel<BN_, BMN_><<<grid, NUM_THREADS, bytes, stream>>>(ma, mb, p, mb2);           \
@@ -1078,11 +1093,12 @@ int tc_lora_project(int which, const void* x, const void* a0, int n0, float s0, 
   return single_grouped_gemm(which, x, a0, m_sizes, ms64, out, M, n0 + (a1 ? n1 : 0), K, E, dtype, dtype, stream, ex);
 }
 
+// out2: rows from n1 on (of the N <= 128) are the rows of a second weight gradient.
 int tc_grouped_gemm_dw_strided(const void* x, int64_t ldx, const void* dy, int64_t ldy, const void* m_sizes, int ms64,
-                               void* out, int64_t M, int N, int K, int E, int dtype, void* ws, size_t ws_bytes,
-                               cudaStream_t stream) {
+                               void* out, void* out2, int n1, int64_t M, int N, int K, int E, int dtype, void* ws,
+                               size_t ws_bytes, cudaStream_t stream) {
   bind_context_once();
-  return dw_grouped_gemm(x, dy, m_sizes, ms64, out, M, N, K, E, dtype, dtype, ws, ws_bytes, stream, false, ldx, ldy);
+  return dw_grouped_gemm(x, dy, m_sizes, ms64, out, M, N, K, E, dtype, dtype, ws, ws_bytes, stream, out2 != nullptr, ldx, ldy, out2, n1);
 }
 
 bool tc_nf4_eligible(const void* x, const void* packed, const void* absmax, const void* out, int64_t M, int N, int K,

@@ -80,6 +80,7 @@ struct DwMaps {
   CUtensorMap dy[DW_BOXES];
   CUtensorMap x[DW_BOXES];
   CUtensorMap out;
+  CUtensorMap out2;  // second output (GemmParams::row_split)
 };
 
 struct DwControl {
@@ -382,6 +383,8 @@ dw_kernel(const __grid_constant__ DwMaps maps, const GemmParams p) {
         named_barrier_sync(1, 128);
         if (epi_tid == 0) {
           tma_store_3d(&maps.out, buf, k0 + c * 64, n0, e);  // rows / columns past N / K are clipped
+          // (a multiple of 8 rows further the staging tile is swizzled as at its start)
+          if (!PAIR && p.row_split) tma_store_3d(&maps.out2, buf + p.row_split * 128, k0 + c * 64, 0, e);
           tma_store_commit();
         }
       }

@@ -39,7 +39,7 @@ SIGNATURES = {
     "moe_grouped_gemm_dw": (_I, [_P, _P, _P, _I, _P, _L, _I, _I, _I, _I, _I, _P, _Z, _P]),
     "moe_grouped_gemm_sum": (_I, [_I, _I, _P, _P, _P, _P, _P, _I, _P, _L, _I, _I, _I, _P]),
     "moe_lora_project": (_I, [_I, _P, _P, _I, _F, _P, _I, _F, _P, _I, _P, _L, _L, _I, _I, _I, _P]),
-    "moe_grouped_gemm_dw_strided": (_I, [_P, _L, _P, _L, _P, _I, _P, _L, _I, _I, _I, _I, _P, _Z, _P]),
+    "moe_grouped_gemm_dw_strided": (_I, [_P, _L, _P, _L, _P, _I, _P, _P, _I, _L, _I, _I, _I, _I, _P, _Z, _P]),
     "moe_gate_up_silu_fwd": (_I, [_P, _P, _P, _P, _I, _P, _L, _I, _I, _I, _I, _P, _Z, _P]),
     "moe_gate_up_silu_fwd_gather": (_I, [_P, _L, _P, _I, _P, _P, _P, _I, _P, _L, _I, _I, _I, _I, _P, _Z, _P]),
     "moe_grouped_gemm_fwd_gather": (_I, [_P, _L, _P, _I, _P, _P, _I, _P, _L, _I, _I, _I, _I, _I, _P, _Z, _P]),

@@ -66,17 +66,19 @@ def lora_project(x: torch.Tensor, a0: torch.Tensor, s0: float, m_sizes: torch.Te
     _lib.check(status, "moe_lora_project")
 
 
-def grouped_gemm_dw_strided(x: torch.Tensor, dy: torch.Tensor, m_sizes: torch.Tensor) -> torch.Tensor:
-    """`grouped_gemm_backward_dw` on operands that may be column slices: w[e] = sum over the rows of e of dy^T x."""
+def grouped_gemm_dw_strided(x: torch.Tensor, dy: torch.Tensor, m_sizes: torch.Tensor, n1: int = 0):
+    """`grouped_gemm_backward_dw` on operands that may be column slices: w[e] = sum over the rows of e of dy^T x.  With
+    `n1` the columns of dy belong to two weights: (E, n1, K) and (E, N - n1, K) are returned."""
     M, K = x.shape
     N, E = dy.shape[1], m_sizes.numel()
-    w = torch.empty((E, N, K), device=x.device, dtype=x.dtype)
+    w = torch.empty((E, n1 or N, K), device=x.device, dtype=x.dtype)
+    w2 = torch.empty((E, N - n1, K), device=x.device, dtype=x.dtype) if n1 else None
     lib = _lib.load()
     m_sizes = _lib.as_index_tensor(m_sizes)
     ws_ptr, ws_bytes = _lib.workspace(x.device, lib.moe_grouped_gemm_workspace_bytes(2, M, N, K, E))
     with torch.cuda.device(x.device):
         status = lib.moe_grouped_gemm_dw_strided(
             _lib.ptr(x), x.stride(0), _lib.ptr(dy), dy.stride(0), _lib.ptr(m_sizes), _lib.int_code(m_sizes.dtype), _lib.ptr(w),
-            M, N, K, E, _lib.float_code(x.dtype), ws_ptr, ws_bytes, _lib.stream_ptr(x.device))
+            _lib.ptr(w2), n1, M, N, K, E, _lib.float_code(x.dtype), ws_ptr, ws_bytes, _lib.stream_ptr(x.device))
     _lib.check(status, "moe_grouped_gemm_dw_strided")
-    return w
+    return (w, w2) if n1 else w
