@@ -107,7 +107,7 @@ MOE_API int moe_set_gemm_path(int path) {
 MOE_API int moe_get_gemm_path(void) { return g_path.load(); }
 
 MOE_API size_t moe_grouped_gemm_workspace_bytes(int, int64_t, int, int, int E) {
-  // per-expert tensor maps derived from m_sizes on the device, and the launch's work-item counter
+  // per-expert tensor maps derived from m_sizes on the device (NF4 and scattered forms)
   return tc_workspace_bytes(E);
 }
 

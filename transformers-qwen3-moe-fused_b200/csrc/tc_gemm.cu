@@ -876,7 +876,7 @@ static int launch_pair_threads(void (*kernel)(KArgs...), int grid, int threads, 
   return cuda_status(cudaLaunchKernelEx(&cfg, kernel, args...));
 }
 
-// dW on tensor cores: per-expert maps are built into `ws`, then one GEMM launch.
+// dW on tensor cores: one launch.  (`ws` is not used; a call without one is refused all the same, as the header says.)
 static int dw_grouped_gemm(const void* x, const void* dy, const void* m_sizes, int ms64, void* out, int64_t M, int N,
                            int K, int E, int dtype_in, int dtype_out, void* ws, size_t ws_bytes, cudaStream_t stream,
                            bool single_cta, int64_t ldx = 0, int64_t ldy = 0, void* out2 = nullptr, int n1 = 0) {

@@ -17,7 +17,7 @@ def _launch(name: str, which: int, a, b, m_sizes, out, M: int, N: int, K: int, E
     lib = _lib.load()
     m_sizes = _lib.as_index_tensor(m_sizes)
     fn = getattr(lib, name)
-    # scratch for the per-expert tensor maps the tensor-core kernels derive from m_sizes
+    # scratch memory that the library's contract asks for (its tensor-core dW refuses a call without it)
     ws_ptr, ws_bytes = _lib.workspace(a.device, lib.moe_grouped_gemm_workspace_bytes(which, M, N, K, E))
     status = fn(
         _lib.ptr(a), _lib.ptr(b), _lib.ptr(m_sizes), _lib.int_code(m_sizes.dtype), _lib.ptr(out),
