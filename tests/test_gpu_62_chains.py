@@ -61,3 +61,19 @@ def test_block_call_equals_composition(cuda, dtype, T, E, k, H, I, norm):
         assert _block_infer(x, logits, gp, odd, dp, k, norm) is None
         out, _ = moe_block_forward(x.view(1, T, H), gw, gp, odd, dp, k, norm)
         assert torch.allclose(out.view(T, H).float(), want.float(), rtol=2e-2, atol=2e-3 * want.float().abs().max().item())
+
+
+@pytest.mark.parametrize("which", range(5))  # tokens, router, gate, up, down
+def test_block_refuses_forward_mode(cuda, which):
+    """No kernel here carries a forward-mode derivative, and `no_grad` does not switch that mode off: a tangent is refused,
+    not dropped."""
+    import torch.autograd.forward_ad as fw
+    from qwen3_moe_fused.moe_block import moe_block_forward
+
+    T, E, k, H, I = 3, 8, 2, 256, 64
+    ts = [torch.ones(s, device=cuda, dtype=torch.bfloat16) for s in ((1, T, H), (E, H), (E, I, H), (E, I, H), (E, H, I))]
+    with torch.no_grad(), fw.dual_level():
+        moe_block_forward(*ts, k)  # inside a level, but without a tangent
+        ts[which] = fw.make_dual(ts[which], torch.ones_like(ts[which]))
+        with pytest.raises(NotImplementedError):
+            moe_block_forward(*ts, k)

@@ -14,6 +14,7 @@ from typing import Optional
 
 import torch
 from torch import nn
+from torch.autograd import forward_ad
 
 from . import _lib
 from .functional import moe_fused_linear
@@ -62,6 +63,12 @@ def route(router_logits: torch.Tensor, num_selected: int, norm_topk_prob: bool, 
     return softmax_topk_autograd(router_logits.contiguous(), num_selected, norm_topk_prob, dtype)
 
 
+def _has_tangent(*tensors) -> bool:
+    """Whether a tensor carries a forward-mode derivative.  Grad mode does not switch forward mode off, and a call that
+    takes addresses would lose the tangent without a word: such tensors go through the autograd functions, which raise."""
+    return any(forward_ad.unpack_dual(t).tangent is not None for t in tensors)
+
+
 def _block_infer(x, router_logits, gate_proj, up_proj, down_proj, k: int, norm_topk_prob: bool) -> Optional[torch.Tensor]:
     """The block after its router GEMM as one call into the library (the same kernels in the same order as the
     composition in `moe_block_forward`); None where that composition has to decide: other dtypes, layouts, extents."""
@@ -102,17 +109,18 @@ def moe_block_forward(hidden_states: torch.Tensor, gate_weight: torch.Tensor, ga
     k = num_selected
     x = hidden_states.reshape(T, H)
     router_logits = torch.nn.functional.linear(x, gate_weight)
-    if not torch.is_grad_enabled() and not GATHER_IN_KERNEL:
+    infer = not torch.is_grad_enabled() and not _has_tangent(x, router_logits, gate_proj, up_proj, down_proj)
+    if infer and not GATHER_IN_KERNEL:
         out = _block_infer(x, router_logits, gate_proj, up_proj, down_proj, k, norm_topk_prob)
         if out is not None:
             return out.view(B, S, H), router_logits
     routing_weights, selected = route(router_logits, k, norm_topk_prob, x.dtype)
     m_sizes, sort_idx, inv_sort_idx = get_expert_counts_and_idx(selected.view(T * k), E)
-    if not torch.is_grad_enabled() and GATHER_IN_KERNEL:
+    if infer and GATHER_IN_KERNEL:
         # gate, up and SiLU-mul in one kernel whose token load gathers the rows straight from the (T, H)
         # tokens (same result bit for bit; the expanded, sorted copy is never written)
         h = gate_up_silu_forward(x.contiguous(), gate_proj, up_proj, m_sizes, row_index=sort_idx, index_div=k)
-    elif not torch.is_grad_enabled():
+    elif infer:
         # inference: gate, up and SiLU-mul in one kernel (same result bit for bit)
         h = gate_up_silu_forward(gather_rows(x.contiguous(), sort_idx, inv_sort_idx, k), gate_proj, up_proj, m_sizes)
     else:
