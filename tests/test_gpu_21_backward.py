@@ -54,3 +54,25 @@ def test_router_backward(cuda, T, E, k, dtype, norm):
         scale = scale / sel.detach().sum(-1, keepdim=True)
     bound = 64 * 2.0 ** -24 * k * scale + 1.01 * ROUND[dtype] * ref.abs() + 1e-30
     assert ((grad.cpu().double() - ref).abs() <= bound).all()
+
+
+def test_combine_backward_twice(cuda):
+    """Gradients taken with create_graph can be differentiated again, in y, the weights and dout."""
+    from qwen3_moe_fused.kernels.routing import combine
+
+    T, k, H = 5, 2, 24
+    gen = torch.Generator().manual_seed(0)
+    inv = torch.randperm(T * k, generator=gen)
+    ii, si = inv.to(torch.int32).to(cuda), torch.argsort(inv).to(torch.int32).to(cuda)
+    ts = [torch.randn(*s, generator=gen) for s in ((T * k, H), (T, k), (T, H))]
+    g = [t.to(cuda).requires_grad_() for t in ts]
+    d = [t.double().requires_grad_() for t in ts]
+
+    def twice(out, y, w, dout):
+        dy, dw = torch.autograd.grad(out, (y, w), dout, create_graph=True)
+        return torch.autograd.grad(dy.square().sum() + dw.square().sum(), (y, w, dout))
+
+    got = twice(combine(g[0], si, ii, g[1]), *g)
+    ref = twice(torch.einsum("tkh,tk->th", d[0][inv].view(T, k, H), d[1]), *d)
+    for a, b in zip(got, ref):  # fp32 sums of up to H * k products of products
+        assert (a.cpu().double() - b).norm() <= 1e-5 * b.norm()

@@ -139,6 +139,12 @@ class Combine(torch.autograd.Function):
         T, k = weights.shape
         dout = dout.contiguous()
         dy = dw = None
+        if torch.is_grad_enabled():  # create_graph: operations that autograd can follow a second time
+            if ctx.needs_input_grad[0]:
+                dy = gather_rows(dout, sort_idx, inv_sort_idx, k) * weights.reshape(-1)[sort_idx.long()].unsqueeze(1)
+            if ctx.needs_input_grad[3]:
+                dw = torch.einsum("tkh,th->tk", y[inv_sort_idx.long()].view(T, k, -1).float(), dout.float()).to(weights.dtype)
+            return dy, None, None, dw
         if ctx.needs_input_grad[0]:
             dy = torch.empty((T * k, y.shape[1]), device=y.device, dtype=y.dtype)
         if ctx.needs_input_grad[3]:
