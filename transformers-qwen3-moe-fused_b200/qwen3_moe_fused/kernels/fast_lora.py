@@ -115,10 +115,10 @@ class FastLora(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, dy):
-        if ctx.fused:
+        if ctx.fused and _lib.load().moe_get_gemm_path() == _lib.PATH_AUTO:  # (may have been switched since the forward)
             return FastLora._backward_fused(ctx, dy)
         Gq, Gqs, Sg, Uq, Uqs, Su, Wq, Wqs, Sw, m_sizes = ctx.custom_saved_tensors
-        x, Ag, Bg, Au, Bu, Aw, Bw, e, g = ctx.saved_tensors
+        x, Ag, Bg, Au, Bu, Aw, Bw, e, g = ctx.saved_tensors[:9]
         dt = x.dtype
         dy = dy.contiguous().to(dt)
 
