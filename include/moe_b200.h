@@ -257,7 +257,8 @@ int moe_block_fwd(const void* x, const void* logits, const void* w_gate, const v
 
 /* The expert MLP with LoRA on dense 16-bit weights, gate / up / down in this order: forward and backward as one call
  * each, built from moe_lora_project, moe_grouped_gemm_sum, moe_grouped_gemm_dw_strided and the SiLU-mul kernels (their
- * conditions apply to every operand).  base (E, I, H), (E, I, H), (E, H, I); a (E, r, in), b (E, out, r).
+ * conditions apply to every operand).  In fp16 a factor's power of two is applied to fp32 accumulators only and has to lie
+ * in 2^-7..2^7 (MOE_ERR_UNSUPPORTED otherwise, nothing enqueued).  base (E, I, H), (E, I, H), (E, H, I); a (E, r, in), b (E, out, r).
  * Forward: e, g, h (M, I), t_gu (M, r_gate + r_up), t_w (M, r_down), y (M, H) are written; all but h and y are what the
  * backward needs.  Backward: e and g are overwritten; dh (M, I), d_gu, d_w (shaped like t_gu, t_w) are scratch; dx may
  * be NULL (not wanted); ws as for moe_grouped_gemm_dw.

@@ -2,6 +2,8 @@
 // forward and backward of the expert MLP with LoRA.  At small sizes the kernels of a chain take less time than a host
 // that goes back to Python between them (a decode step: 45 us of kernels, 190 us of host); nothing here touches device
 // memory or changes what is launched.
+#include <cmath>
+
 #include "common.cuh"
 
 using namespace moe;
@@ -49,6 +51,28 @@ bool block_shape_ok(int64_t T, int H, int I, int E, int k, int dtype) {
          T * k <= 0x7fffffffLL - 1024 && is_float_dtype(dtype);
 }
 
+// The factor s of a LoRA product as thin * 2^log2.  `thin` goes onto the fp32 accumulator of the thin factor (t = s x A^T,
+// d = s dy B), which is then rounded to 16 bits; 2^log2 onto the accumulators of the products with the thin factor.
+// bf16 has fp32's range: all of s in one go.  In fp16 it would cost thin factors small ones their low bits or large ones
+// their range: 1 <= |thin| < 2, and +-1 for powers of two, so that the thin factors are held as they are.
+struct Factor {
+  float thin = 1.f;
+  int log2 = 0;
+  Factor(float s, int dtype) : thin(s) {
+    if (dtype != MOE_F16 || s == 0.f || !std::isfinite(s)) return;
+    thin = 2.f * std::frexp(s, &log2);
+    --log2;
+  }
+  float pow2() const { return std::ldexp(1.f, log2); }
+};
+
+// Whether the accumulators can be rescaled by the factors (by at most 2^15 between two products).
+bool factors_ok(const Factor* f) {
+  for (int i = 0; i < 3; ++i)
+    if (f[i].log2 < -7 || f[i].log2 > 7) return false;
+  return true;
+}
+
 }  // namespace
 
 MOE_API size_t moe_block_fwd_scratch_bytes(int64_t T, int H, int I, int E, int k, int dtype) {
@@ -86,21 +110,24 @@ MOE_API int moe_lora_mlp_fwd(const moe_lora_weights* w, const void* x, const voi
   if (M <= 0 || H <= 0 || I <= 0 || rg <= 0 || ru <= 0 || rw <= 0) return MOE_ERR_SHAPE;
   const int64_t ld = rg + ru;
   uint8_t* t_u = (uint8_t*)t_gu + (size_t)rg * dtype_size(dtype);
-  auto sum2 = [&](const void* x0, const void* w0, int k0, const void* t, int64_t ldt, const void* b, int r, void* out, int N) {
+  const Factor f[3] = {{w->scale[0], dtype}, {w->scale[1], dtype}, {w->scale[2], dtype}};
+  if (!factors_ok(f)) return MOE_ERR_UNSUPPORTED;
+  auto sum2 = [&](const void* x0, int i, int k0, const void* t, int64_t ldt, void* out, int N) {
     const void* xs[2] = {x0, t};
-    const void* ws[2] = {w0, b};
+    const void* ws[2] = {w->base[i], w->b[i]};
     const int64_t lds[2] = {k0, ldt};
-    const int ks[2] = {k0, r};
-    return moe_grouped_gemm_sum(0, 2, xs, lds, ws, ks, m_sizes, msd, out, M, N, E, dtype, stream);
+    const int ks[2] = {k0, w->rank[i]};
+    const int log2_scale[2] = {0, f[i].log2};
+    return grouped_gemm_sum_scaled(0, 2, xs, lds, ws, ks, log2_scale, m_sizes, msd, out, M, N, E, dtype, stream);
   };
   int st;
-  // thin factors of the LoRA products, already scaled: gate and up side by side (x is read once), down
-  if ((st = moe_lora_project(0, x, w->a[0], rg, w->scale[0], w->a[1], ru, w->scale[1], m_sizes, msd, t_gu, ld, M, H, E, dtype, stream)) != MOE_OK) return st;
-  if ((st = sum2(x, w->base[0], H, t_gu, ld, w->b[0], rg, e, I)) != MOE_OK) return st;
-  if ((st = sum2(x, w->base[1], H, t_u, ld, w->b[1], ru, g, I)) != MOE_OK) return st;
+  // thin factors of the LoRA products: gate and up side by side (x is read once), down
+  if ((st = moe_lora_project(0, x, w->a[0], rg, f[0].thin, w->a[1], ru, f[1].thin, m_sizes, msd, t_gu, ld, M, H, E, dtype, stream)) != MOE_OK) return st;
+  if ((st = sum2(x, 0, H, t_gu, ld, e, I)) != MOE_OK) return st;
+  if ((st = sum2(x, 1, H, t_u, ld, g, I)) != MOE_OK) return st;
   if ((st = moe_silu_mul_fwd(e, g, h, M * I, dtype, stream)) != MOE_OK) return st;
-  if ((st = moe_lora_project(0, h, w->a[2], rw, w->scale[2], nullptr, 0, 1.f, m_sizes, msd, t_w, rw, M, I, E, dtype, stream)) != MOE_OK) return st;
-  return sum2(h, w->base[2], I, t_w, rw, w->b[2], rw, y, H);
+  if ((st = moe_lora_project(0, h, w->a[2], rw, f[2].thin, nullptr, 0, 1.f, m_sizes, msd, t_w, rw, M, I, E, dtype, stream)) != MOE_OK) return st;
+  return sum2(h, 2, I, t_w, rw, y, H);
 }
 
 MOE_API int moe_lora_mlp_bwd(const moe_lora_weights* w, const moe_lora_grads* grads, const void* dy, const void* x,
@@ -114,37 +141,42 @@ MOE_API int moe_lora_mlp_bwd(const moe_lora_weights* w, const moe_lora_grads* gr
   const size_t off = (size_t)rg * dtype_size(dtype);
   const uint8_t* t_u = (const uint8_t*)t_gu + off;
   uint8_t* d_u = (uint8_t*)d_gu + off;
-  auto dw = [&](const void* x_, int64_t ldx, int K, const void* dy_, int64_t ldy, int N, void* out) {
-    return moe_grouped_gemm_dw_strided(x_, ldx, dy_, ldy, m_sizes, msd, out, nullptr, 0, M, N, K, E, dtype, ws, ws_bytes, stream);
+  const Factor f[3] = {{w->scale[0], dtype}, {w->scale[1], dtype}, {w->scale[2], dtype}};
+  if (!factors_ok(f)) return MOE_ERR_UNSUPPORTED;
+  auto dw = [&](int i, const void* x_, int64_t ldx, int K, const void* dy_, int64_t ldy, int N, void* out) {
+    return grouped_gemm_dw_scaled(x_, ldx, dy_, ldy, m_sizes, msd, out, nullptr, 0, f[i].pow2(), 1.f, M, N, K, E, dtype, ws,
+                                  ws_bytes, stream);
   };
   int st;
-  if ((st = moe_lora_project(1, dy, w->b[2], rw, w->scale[2], nullptr, 0, 1.f, m_sizes, msd, d_w, rw, M, H, E, dtype, stream)) != MOE_OK) return st;
+  if ((st = moe_lora_project(1, dy, w->b[2], rw, f[2].thin, nullptr, 0, 1.f, m_sizes, msd, d_w, rw, M, H, E, dtype, stream)) != MOE_OK) return st;
   {
     const void* xs[2] = {dy, d_w};
     const void* wt[2] = {w->base[2], w->a[2]};
     const int64_t lds[2] = {H, rw};
     const int ks[2] = {H, rw};
-    if ((st = moe_grouped_gemm_sum(1, 2, xs, lds, wt, ks, m_sizes, msd, dh, M, I, E, dtype, stream)) != MOE_OK) return st;
+    const int log2_scale[2] = {0, f[2].log2};
+    if ((st = grouped_gemm_sum_scaled(1, 2, xs, lds, wt, ks, log2_scale, m_sizes, msd, dh, M, I, E, dtype, stream)) != MOE_OK) return st;
   }
   // dh, e, g become h, de, dg
   if ((st = moe_silu_mul_bwd_inplace(dh, e, g, M * I, dtype, stream)) != MOE_OK) return st;
-  if ((st = dw(dh, I, I, d_w, rw, rw, grads->da[2])) != MOE_OK) return st;
-  if ((st = dw(t_w, rw, rw, dy, H, H, grads->db[2])) != MOE_OK) return st;
-  if ((st = moe_lora_project(1, e, w->b[0], rg, w->scale[0], nullptr, 0, 1.f, m_sizes, msd, d_gu, ld, M, I, E, dtype, stream)) != MOE_OK) return st;
-  if ((st = moe_lora_project(1, g, w->b[1], ru, w->scale[1], nullptr, 0, 1.f, m_sizes, msd, d_u, ld, M, I, E, dtype, stream)) != MOE_OK) return st;
+  if ((st = dw(2, dh, I, I, d_w, rw, rw, grads->da[2])) != MOE_OK) return st;
+  if ((st = dw(2, t_w, rw, rw, dy, H, H, grads->db[2])) != MOE_OK) return st;
+  if ((st = moe_lora_project(1, e, w->b[0], rg, f[0].thin, nullptr, 0, 1.f, m_sizes, msd, d_gu, ld, M, I, E, dtype, stream)) != MOE_OK) return st;
+  if ((st = moe_lora_project(1, g, w->b[1], ru, f[1].thin, nullptr, 0, 1.f, m_sizes, msd, d_u, ld, M, I, E, dtype, stream)) != MOE_OK) return st;
   if (rg + ru <= 128) {  // both gradients of a from one read of x
-    if ((st = moe_grouped_gemm_dw_strided(x, H, d_gu, ld, m_sizes, msd, grads->da[0], grads->da[1], rg, M, rg + ru, H, E, dtype, ws,
-                                          ws_bytes, stream)) != MOE_OK) return st;
+    if ((st = grouped_gemm_dw_scaled(x, H, d_gu, ld, m_sizes, msd, grads->da[0], grads->da[1], rg, f[0].pow2(), f[1].pow2(), M,
+                                     rg + ru, H, E, dtype, ws, ws_bytes, stream)) != MOE_OK) return st;
   } else {
-    if ((st = dw(x, H, H, d_gu, ld, rg, grads->da[0])) != MOE_OK) return st;
-    if ((st = dw(x, H, H, d_u, ld, ru, grads->da[1])) != MOE_OK) return st;
+    if ((st = dw(0, x, H, H, d_gu, ld, rg, grads->da[0])) != MOE_OK) return st;
+    if ((st = dw(1, x, H, H, d_u, ld, ru, grads->da[1])) != MOE_OK) return st;
   }
-  if ((st = dw(t_gu, ld, rg, e, I, I, grads->db[0])) != MOE_OK) return st;
-  if ((st = dw(t_u, ld, ru, g, I, I, grads->db[1])) != MOE_OK) return st;
+  if ((st = dw(0, t_gu, ld, rg, e, I, I, grads->db[0])) != MOE_OK) return st;
+  if ((st = dw(1, t_u, ld, ru, g, I, I, grads->db[1])) != MOE_OK) return st;
   if (!dx) return MOE_OK;
   const void* xs[4] = {e, d_gu, g, d_u};
   const void* wt[4] = {w->base[0], w->a[0], w->base[1], w->a[1]};
   const int64_t lds[4] = {I, ld, I, ld};
   const int ks[4] = {I, rg, I, ru};
-  return moe_grouped_gemm_sum(1, 4, xs, lds, wt, ks, m_sizes, msd, dx, M, H, E, dtype, stream);
+  const int log2_scale[4] = {0, f[0].log2, 0, f[1].log2};
+  return grouped_gemm_sum_scaled(1, 4, xs, lds, wt, ks, log2_scale, m_sizes, msd, dx, M, H, E, dtype, stream);
 }

@@ -56,6 +56,15 @@ inline int sm_count() {
   return cached[dev];
 }
 
+// moe_grouped_gemm_sum whose product i counts 2^log2_scale[i] times (null: once; at most 2^15 between any two), and
+// moe_grouped_gemm_dw_strided whose gradients are multiplied by alpha / alpha2 ahead of their rounding (gemm_api.cu).
+int grouped_gemm_sum_scaled(int which, int n, const void* const* x, const int64_t* ldx, const void* const* w, const int* K,
+                            const int* log2_scale, const void* m_sizes, int msd, void* y, int64_t M, int N, int E, int dtype,
+                            void* stream);
+int grouped_gemm_dw_scaled(const void* x, int64_t ldx, const void* dy, int64_t ldy, const void* m_sizes, int msd, void* w,
+                           void* w2, int n1, float alpha, float alpha2, int64_t M, int N, int K, int E, int dtype, void* ws,
+                           size_t ws_bytes, void* stream);
+
 }  // namespace moe
 
 // Run `body` with `T` bound to the C++ type of a floating dtype code.

@@ -31,13 +31,13 @@ int tc_grouped_gemm_gather(const void* x, int64_t x_rows, const int* row_index, 
                            const void* m_sizes, int ms64, void* y, int64_t M, int N, int K, int E, int dtype_in,
                            int dtype_out, void* ws, size_t ws_bytes, cudaStream_t stream);
 int tc_grouped_gemm_sum(int which, int n, const void* const* x, const int64_t* ldx, const void* const* w, const int* K,
-                        const void* m_sizes, int ms64, void* out, int64_t M, int N, int E, int dtype, cudaStream_t stream);
+                        const int* log2_scale, const void* m_sizes, int ms64, void* out, int64_t M, int N, int E, int dtype, cudaStream_t stream);
 int tc_lora_project(int which, const void* x, const void* a0, int n0, float s0, const void* a1, int n1, float s1,
                     const void* m_sizes, int ms64, void* out, int ld_out, int64_t M, int K, int E, int dtype,
                     cudaStream_t stream);
 int tc_grouped_gemm_dw_strided(const void* x, int64_t ldx, const void* dy, int64_t ldy, const void* m_sizes, int ms64,
-                               void* out, void* out2, int n1, int64_t M, int N, int K, int E, int dtype, void* ws,
-                               size_t ws_bytes, cudaStream_t stream);
+                               void* out, void* out2, int n1, float alpha, float alpha2, int64_t M, int N, int K, int E,
+                               int dtype, void* ws, size_t ws_bytes, cudaStream_t stream);
 int tc_read_error(int* flag_out, bool clear);
 size_t tc_workspace_bytes(int E);
 int tc_read_late_values(int* out);
@@ -228,9 +228,9 @@ MOE_API int moe_grouped_gemm_fwd_gather(const void* x, int64_t x_rows, const int
 }
 
 // Contractions of several (activation, weight) pairs summed in one accumulator.  Tensor-core CTA-pair kernel only.
-MOE_API int moe_grouped_gemm_sum(int which, int n, const void* const* x, const int64_t* ldx, const void* const* w,
-                                 const int* K, const void* m_sizes, int msd, void* y, int64_t M, int N, int E, int dtype,
-                                 void* stream) {
+int moe::grouped_gemm_sum_scaled(int which, int n, const void* const* x, const int64_t* ldx, const void* const* w, const int* K,
+                                 const int* log2_scale, const void* m_sizes, int msd, void* y, int64_t M, int N, int E,
+                                 int dtype, void* stream) {
   if ((which != 0 && which != 1) || n < 1 || n > 4) return MOE_ERR_SHAPE;
   if (!x || !ldx || !w || !K) return MOE_ERR_NULL;
   for (int i = 0; i < n; ++i) {
@@ -244,7 +244,13 @@ MOE_API int moe_grouped_gemm_sum(int which, int n, const void* const* x, const i
   if (path == MOE_PATH_SIMT || path == MOE_PATH_TC_SINGLE || N < 192 || ((uintptr_t)y & 15)) return MOE_ERR_UNSUPPORTED;
   for (int i = 0; i < n; ++i)
     if (ldx[i] % 8 || !tc_eligible(which, x[i], w[i], y, M, N, K[i], E, dtype, dtype)) return MOE_ERR_UNSUPPORTED;
-  return tc_grouped_gemm_sum(which, n, x, ldx, w, K, m_sizes, msd == MOE_I64, y, M, N, E, dtype, (cudaStream_t)stream);
+  return tc_grouped_gemm_sum(which, n, x, ldx, w, K, log2_scale, m_sizes, msd == MOE_I64, y, M, N, E, dtype, (cudaStream_t)stream);
+}
+
+MOE_API int moe_grouped_gemm_sum(int which, int n, const void* const* x, const int64_t* ldx, const void* const* w,
+                                 const int* K, const void* m_sizes, int msd, void* y, int64_t M, int N, int E, int dtype,
+                                 void* stream) {
+  return grouped_gemm_sum_scaled(which, n, x, ldx, w, K, nullptr, m_sizes, msd, y, M, N, E, dtype, stream);
 }
 
 MOE_API int moe_lora_project(int which, const void* x, const void* a0, int n0, float s0, const void* a1, int n1, float s1,
@@ -266,9 +272,9 @@ MOE_API int moe_lora_project(int which, const void* x, const void* a0, int n0, f
                          (cudaStream_t)stream);
 }
 
-MOE_API int moe_grouped_gemm_dw_strided(const void* x, int64_t ldx, const void* dy, int64_t ldy, const void* m_sizes,
-                                        int msd, void* w, void* w2, int n1, int64_t M, int N, int K, int E, int dtype,
-                                        void* ws, size_t ws_bytes, void* stream) {
+int moe::grouped_gemm_dw_scaled(const void* x, int64_t ldx, const void* dy, int64_t ldy, const void* m_sizes, int msd, void* w,
+                                void* w2, int n1, float alpha, float alpha2, int64_t M, int N, int K, int E, int dtype,
+                                void* ws, size_t ws_bytes, void* stream) {
   if (!is_float_dtype(dtype) || !is_int_dtype(msd)) return MOE_ERR_DTYPE;
   if (M < 0 || N < 0 || K < 0 || E <= 0 || M > 0x7fffffffLL || ldx < K || ldy < N) return MOE_ERR_SHAPE;
   if (!m_sizes) return MOE_ERR_NULL;
@@ -285,8 +291,14 @@ MOE_API int moe_grouped_gemm_dw_strided(const void* x, int64_t ldx, const void* 
   const int path = g_path.load(std::memory_order_relaxed);
   if (w2 && (N > 128 || n1 % 8 || (((uintptr_t)w | (uintptr_t)w2) & 15))) return MOE_ERR_UNSUPPORTED;
   if (path == MOE_PATH_SIMT || ldx % 8 || ldy % 8 || !tc_eligible(2, x, dy, w, M, N, K, E, dtype, dtype)) return MOE_ERR_UNSUPPORTED;
-  return tc_grouped_gemm_dw_strided(x, ldx, dy, ldy, m_sizes, msd == MOE_I64, w, w2, n1, M, N, K, E, dtype, ws, ws_bytes,
-                                    (cudaStream_t)stream);
+  return tc_grouped_gemm_dw_strided(x, ldx, dy, ldy, m_sizes, msd == MOE_I64, w, w2, n1, alpha, alpha2, M, N, K, E, dtype, ws,
+                                    ws_bytes, (cudaStream_t)stream);
+}
+
+MOE_API int moe_grouped_gemm_dw_strided(const void* x, int64_t ldx, const void* dy, int64_t ldy, const void* m_sizes,
+                                        int msd, void* w, void* w2, int n1, int64_t M, int N, int K, int E, int dtype,
+                                        void* ws, size_t ws_bytes, void* stream) {
+  return grouped_gemm_dw_scaled(x, ldx, dy, ldy, m_sizes, msd, w, w2, n1, 1.f, 1.f, M, N, K, E, dtype, ws, ws_bytes, stream);
 }
 
 static int run_scattered(int which, const void* x, const void* w, const void* group_sizes, int msd,

@@ -310,6 +310,21 @@ __device__ __forceinline__ void umma_f16_pair(uint32_t tmem_d, uint64_t desc_a, 
       ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
       : "memory");
 }
+// D[tmem] = D * 2^-SHIFT + A * B: the accumulator is rescaled by the MMA itself (exact in fp32).
+template <int SHIFT>
+__device__ __forceinline__ void umma_f16_pair_rescale(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc) {
+  static_assert(SHIFT >= 1 && SHIFT <= 15, "range of the instruction's immediate");
+  asm volatile(
+      "{\n\t.reg .pred p;\n\tsetp.eq.b32 p, 0, 0;\n\t"
+      "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p, %4;\n\t}"
+      ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "n"(SHIFT)
+      : "memory");
+}
+template <int MAX = 15>
+__device__ __forceinline__ void umma_f16_pair_rescale(int shift, uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc) {
+  if (shift == MAX) umma_f16_pair_rescale<MAX>(tmem_d, desc_a, desc_b, idesc);
+  else if constexpr (MAX > 1) umma_f16_pair_rescale<MAX - 1>(shift, tmem_d, desc_a, desc_b, idesc);
+}
 // One arrival on the barrier at the same shared-memory offset in every CTA of `cta_mask`,
 // once all MMAs issued so far have completed.
 __device__ __forceinline__ void umma_commit_pair(uint64_t* bar, uint16_t cta_mask) {

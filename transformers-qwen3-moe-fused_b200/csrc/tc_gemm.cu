@@ -11,6 +11,7 @@
 // buffered in TMEM so the epilogue of tile i overlaps the main loop of tile i+1.
 // No tile ever crosses an expert boundary on the store side: an M tile starts at a group's
 // first row and rows past the group's end are computed but not stored.
+#include <cmath>
 #include <cstdio>
 #include <mutex>
 #include <cstdlib>
@@ -44,8 +45,9 @@ struct GemmParams {
   const int* weight_index = nullptr;  // weight slice of each group (null: group e uses slice e)
   int stages = 0;               // CTA-pair forward / dX: depth of the operand ring
   int ld_out = 0;               // single-CTA forward / dX: row pitch of the output (0: N)
-  float alpha[2] = {1.f, 1.f};  // single-CTA forward / dX: factors of the columns before / from b_split on
-  int scaled = 0;               //   (applied to the fp32 accumulator, when set)
+  float alpha[2] = {1.f, 1.f};  // factors of the fp32 accumulator.  Single-CTA forward / dX: columns before / from b_split on;
+                                // dW: rows before / from row_split on; CTA pairs, several operand pairs: alpha[0]
+  int scaled = 0;               //   (single-CTA forward / dX, dW: applied when set)
   int b_split = 0;              // single-CTA forward: columns taken from the first weight (0: there is one weight)
   int row_split = 0;            // single-CTA dW: rows from here on go to the second output (0: there is one output)
   int staged = 0;               // CTA-pair forward / dX: 16-bit output that may leave by TMA
@@ -771,6 +773,7 @@ struct PairOperand {
   const void* w;
   int K;
   int64_t pitch;
+  int log2_scale = 0;  // the product counts 2^log2_scale times
 };
 
 static int fill_pair_operand(tc::PairMaps& maps, int i, int which, const PairOperand& o, int64_t M, int N, int n_weights,
@@ -810,6 +813,13 @@ static int pair_grouped_gemm(int which, const PairOperand* ops, int n_ops, const
                              int64_t x_rows = 0) {
   using namespace tc;
   if ((which != 0 && which != 1) || n_ops < 1 || n_ops > PAIR_MAX_SEGS) return MOE_ERR_UNSUPPORTED;
+  PairOperand sorted[PAIR_MAX_SEGS];  // by rising log2_scale, see "Segments" at the kernel
+  for (int i = 0; i < n_ops; ++i) {
+    int j = i;
+    for (; j > 0 && sorted[j - 1].log2_scale > ops[i].log2_scale; --j) sorted[j] = sorted[j - 1];
+    sorted[j] = ops[i];
+  }
+  ops = sorted;
   const bool gather = row_index != nullptr;
   if (gather && (which != 0 || n_ops != 1 || index_div <= 0 || x_rows <= 0 || x_rows > 0x7fffffffLL)) return MOE_ERR_UNSUPPORTED;
   if (n_weights <= 0) n_weights = E;
@@ -827,6 +837,11 @@ static int pair_grouped_gemm(int which, const PairOperand* ops, int n_ops, const
   int st;
   for (int i = 0; i < n_ops; ++i)
     if ((st = fill_pair_operand(maps, i, which, ops[i], gather ? x_rows : M, N, n_weights, dtype_in)) != MOE_OK) return st;
+  for (int i = 1; i < n_ops; ++i) {
+    maps.shift[i] = ops[i].log2_scale - ops[i - 1].log2_scale;
+    if (maps.shift[i] > 15) return MOE_ERR_UNSUPPORTED;  // the MMA's immediate
+  }
+  p.alpha[0] = ldexpf(1.f, ops[n_ops - 1].log2_scale);
   // gathered token rows: one-row boxes (for gather4) over the x_rows token rows
   if (gather && (st = make_map(&maps.x[0], dtype_in, ops[0].x, (uint64_t)ops[0].K, (uint64_t)x_rows, 0, 1)) != MOE_OK) return st;
   p.idesc = make_idesc(dtype_in == MOE_BF16 ? 1 : 0, which == 1, 0, 256, 0);  // N field is filled per tile
@@ -879,7 +894,8 @@ static int launch_pair_threads(void (*kernel)(KArgs...), int grid, int threads, 
 // dW on tensor cores: one launch.  (`ws` is not used; a call without one is refused all the same, as the header says.)
 static int dw_grouped_gemm(const void* x, const void* dy, const void* m_sizes, int ms64, void* out, int64_t M, int N,
                            int K, int E, int dtype_in, int dtype_out, void* ws, size_t ws_bytes, cudaStream_t stream,
-                           bool single_cta, int64_t ldx = 0, int64_t ldy = 0, void* out2 = nullptr, int n1 = 0) {
+                           bool single_cta, int64_t ldx = 0, int64_t ldy = 0, void* out2 = nullptr, int n1 = 0,
+                           float alpha = 1.f, float alpha2 = 1.f) {
   using namespace tc;
   if (!ws_usable(ws, ws_bytes, E)) return MOE_ERR_WORKSPACE;
   GemmParams p;
@@ -896,6 +912,8 @@ static int dw_grouped_gemm(const void* x, const void* dy, const void* m_sizes, i
   const bool staged = dtype_out != MOE_F32;
   if (out2 != nullptr && (!staged || N > 128 || n1 <= 0 || n1 >= N || n1 % 8)) return MOE_ERR_UNSUPPORTED;
   p.row_split = out2 != nullptr ? n1 : 0;
+  p.alpha[0] = alpha; p.alpha[1] = alpha2;
+  p.scaled = alpha != 1.f || (out2 != nullptr && alpha2 != 1.f);
   if (staged && (st = make_map(&maps.out, dtype_out, out, (uint64_t)K, (uint64_t)(out2 ? n1 : N), (uint64_t)E, 128)) != MOE_OK) return st;
   if (out2 && (st = make_map(&maps.out2, dtype_out, out2, (uint64_t)K, (uint64_t)(N - n1), (uint64_t)E, (uint32_t)(128 - n1))) != MOE_OK) return st;
   const int tables = 2 * (E + 1) * 4 + (int)sizeof(DwControl) + 1024 + 2 * 128 * 128;
@@ -1074,11 +1092,12 @@ int tc_grouped_gemm_scattered(int which, const void* a, const void* b, const voi
 }
 
 // y = sum_i x_i W_i^T (which = 0) or sum_i x_i W_i (which = 1), the contractions of n operand pairs in one accumulator.
+// Product i counts 2^log2_scale[i] times (null: once).
 int tc_grouped_gemm_sum(int which, int n, const void* const* x, const int64_t* ldx, const void* const* w, const int* K,
-                        const void* m_sizes, int ms64, void* out, int64_t M, int N, int E, int dtype, cudaStream_t stream) {
+                        const int* log2_scale, const void* m_sizes, int ms64, void* out, int64_t M, int N, int E, int dtype, cudaStream_t stream) {
   bind_context_once();
   PairOperand ops[tc::PAIR_MAX_SEGS];
-  for (int i = 0; i < n; ++i) ops[i] = PairOperand{x[i], w[i], K[i], ldx[i]};
+  for (int i = 0; i < n; ++i) ops[i] = PairOperand{x[i], w[i], K[i], ldx[i], log2_scale ? log2_scale[i] : 0};
   return pair_grouped_gemm(which, ops, n, m_sizes, ms64, out, M, N, E, dtype, dtype, nullptr, 0, stream);
 }
 
@@ -1093,12 +1112,13 @@ int tc_lora_project(int which, const void* x, const void* a0, int n0, float s0, 
   return single_grouped_gemm(which, x, a0, m_sizes, ms64, out, M, n0 + (a1 ? n1 : 0), K, E, dtype, dtype, stream, ex);
 }
 
-// out2: rows from n1 on (of the N <= 128) are the rows of a second weight gradient.
+// out2: rows from n1 on (of the N <= 128) are the rows of a second weight gradient.  alpha, alpha2: factors of the two.
 int tc_grouped_gemm_dw_strided(const void* x, int64_t ldx, const void* dy, int64_t ldy, const void* m_sizes, int ms64,
-                               void* out, void* out2, int n1, int64_t M, int N, int K, int E, int dtype, void* ws,
-                               size_t ws_bytes, cudaStream_t stream) {
+                               void* out, void* out2, int n1, float alpha, float alpha2, int64_t M, int N, int K, int E,
+                               int dtype, void* ws, size_t ws_bytes, cudaStream_t stream) {
   bind_context_once();
-  return dw_grouped_gemm(x, dy, m_sizes, ms64, out, M, N, K, E, dtype, dtype, ws, ws_bytes, stream, out2 != nullptr, ldx, ldy, out2, n1);
+  return dw_grouped_gemm(x, dy, m_sizes, ms64, out, M, N, K, E, dtype, dtype, ws, ws_bytes, stream, out2 != nullptr, ldx, ldy, out2, n1,
+                         alpha, alpha2);
 }
 
 bool tc_nf4_eligible(const void* x, const void* packed, const void* absmax, const void* out, int64_t M, int N, int K,

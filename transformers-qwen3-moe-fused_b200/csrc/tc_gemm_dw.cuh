@@ -347,6 +347,11 @@ dw_kernel(const __grid_constant__ DwMaps maps, const GemmParams p) {
 #pragma unroll
           for (int i = 0; i < 64; ++i) v[i] = 0;
         }
+        if (p.scaled) {
+          const float f = p.row_split && row >= p.row_split ? p.alpha[1] : p.alpha[0];
+#pragma unroll
+          for (int i = 0; i < 64; ++i) v[i] = __float_as_uint(__uint_as_float(v[i]) * f);
+        }
         if (!staged) {
           // fp32 output: straight from registers
           const int n = n0 + row;

@@ -41,8 +41,10 @@
 // group leaves by TMA; the group's last round, if it is partial, is copied row by row from the staging tile.
 //
 // Segments.  The contraction may run over several (weight, activation) operand pairs into one accumulator:
-//     y[t,:] = sum_i  W_i[e] x_i[t,:]
-// (base weight + LoRA product, or gate + up gradients): see PairMaps.
+//     y[t,:] = sum_i  2^k_i W_i[e] x_i[t,:]
+// (base weight + LoRA product, or gate + up gradients): see PairMaps.  The powers of two never touch a 16-bit operand:
+// segments are ordered by rising k_i, the first MMA of a segment rescales the accumulator by 2^(k_{i-1} - k_i), and the
+// epilogue multiplies by 2^k of the last one, all exact in fp32.
 #pragma once
 
 namespace moe {
@@ -83,6 +85,7 @@ struct PairMaps {
   CUtensorMap out;                // 16-bit outputs: boxes of 32 rows
   int kb[PAIR_MAX_SEGS];
   int last_steps[PAIR_MAX_SEGS];  // MMA steps of 16 in the last block (MULTI)
+  int shift[PAIR_MAX_SEGS];       // the accumulator is multiplied by 2^-shift ahead of the segment (MULTI; 0 for the first)
   int n_seg;
 };
 
@@ -130,10 +133,12 @@ __device__ __forceinline__ void store_clipped_rows(const uint8_t* buf, uint8_t* 
 // Rows: with `out` == nullptr `my` is the group's own map and clips them too; otherwise `my` covers the whole
 // output and a round that reaches past `t_end` is copied from the staging tile instead.
 // Called by the 128 epilogue threads (warps 2..5); `staging` holds 4 * PAIR_STAGING_BYTES.
+// SCALED: the accumulator is multiplied by `scale` first.
+template <bool SCALED = false>
 __device__ __forceinline__ void pair_store_tile_staged(uint8_t* staging, uint32_t& chunk_it, uint32_t taddr, int n_mma,
                                                        int quarter, int lane, int epi_tid, bool is_bf16,
                                                        const CUtensorMap* my, int n_cta, int t0, int N,
-                                                       uint8_t* out = nullptr, int t_end = 0) {
+                                                       uint8_t* out = nullptr, int t_end = 0, float scale = 1.f) {
   const int half = quarter >> 1;
   const int chunk = 4 * (quarter & 1) + (lane >> 3);  // 16-byte chunk of the 128-byte staging row
 #pragma unroll 1
@@ -145,6 +150,13 @@ __device__ __forceinline__ void pair_store_tile_staged(uint8_t* staging, uint32_
     tmem_ld_16x256b_x4(taddr + c, lo);
     tmem_ld_16x256b_x4(taddr + c + (16u << 16), hi);
     tmem_ld_wait();
+    if constexpr (SCALED) {
+#pragma unroll
+      for (int i = 0; i < 16; ++i) {
+        lo[i] = __float_as_uint(__uint_as_float(lo[i]) * scale);
+        hi[i] = __float_as_uint(__uint_as_float(hi[i]) * scale);
+      }
+    }
     uint8_t* tile_buf = buf + half * PAIR_STAGING_BYTES;
 #pragma unroll
     for (int g = 0; g < 4; ++g) {
@@ -577,7 +589,8 @@ pair_fwd_kernel(const __grid_constant__ PairMaps maps, const GemmParams p) {
         const uint32_t d_tail = tmem_base + (par ? PAIR_TOKENS - PAIR_TAIL : PAIR_TOKENS);
         // One block of 64 of the contraction.  Compiled with and without the tail MMAs, and with all steps or a
         // counted number of them: a test between the MMAs of one block costs the issuing thread a quarter of its rate.
-        auto block = [&](auto has_tail, auto all_steps, int steps, bool first) {
+        // `shift`: the accumulator is rescaled by 2^-shift on the way (counted form only).
+        auto block = [&](auto has_tail, auto all_steps, int steps, bool first, int shift = 0) {
           if (!mbar_wait_cluster(&ctl->full[s], ph, abort_flag, PW_FULL)) { ok = false; return; }
           tc_fence_after_sync();
           const uint32_t sa = smem_u32(smem + s * STAGE_BYTES);
@@ -588,6 +601,9 @@ pair_fwd_kernel(const __grid_constant__ PairMaps maps, const GemmParams p) {
           auto step = [&](int k, uint32_t d, uint64_t desc_b, uint32_t idesc) {
             const uint64_t b_adv = (uint64_t)((k * UMMA_K * 2) >> 4);
             const uint64_t a_adv = W_MN ? (uint64_t)((k * UMMA_K * 128) >> 4) : b_adv;
+            if constexpr (MULTI && !decltype(all_steps)::value) {
+              if (shift != 0 && k == 0) { umma_f16_pair_rescale(shift, d, da, desc_b, idesc); return; }
+            }
             umma_f16_pair(d, da + a_adv, desc_b + b_adv, idesc, !first || k != 0);
           };
           if constexpr (decltype(all_steps)::value) {
@@ -612,8 +628,13 @@ pair_fwd_kernel(const __grid_constant__ PairMaps maps, const GemmParams p) {
             // (one operand pair: rows past the contraction's end are zeros in both operands and cost nothing to add)
             const bool partial = MULTI && maps.last_steps[i] < BK / UMMA_K;
             const int full_blocks = maps.kb[i] - (partial ? 1 : 0);
-            for (int kb = 0; kb < full_blocks && ok; ++kb) block(has_tail, std::true_type{}, BK / UMMA_K, (i | kb) == 0);
-            if (MULTI && partial && ok) block(has_tail, std::false_type{}, maps.last_steps[i], (i | full_blocks) == 0);
+            int kb = 0;
+            if (MULTI && maps.shift[i] != 0) {
+              block(has_tail, std::false_type{}, full_blocks > 0 ? BK / UMMA_K : maps.last_steps[i], false, maps.shift[i]);
+              kb = 1;
+            }
+            for (; kb < full_blocks && ok; ++kb) block(has_tail, std::true_type{}, BK / UMMA_K, (i | kb) == 0);
+            if (MULTI && partial && kb < maps.kb[i] && ok) block(has_tail, std::false_type{}, maps.last_steps[i], (i | kb) == 0);
           }
         };
         if (t.n_tail) k_loop(std::true_type{}); else k_loop(std::false_type{});
@@ -656,8 +677,8 @@ pair_fwd_kernel(const __grid_constant__ PairMaps maps, const GemmParams p) {
           pair_store_tile_gate_up(staging, chunk_it, taddr, n_cols, quarter, lane, epi_tid, is_bf16, my,
                                   t.n0 + (int)rank * 64, tok0, p.N, reinterpret_cast<uint8_t*>(p.out), t.t_end);
         } else if (staged) {
-          pair_store_tile_staged(staging, chunk_it, taddr, n_cols, quarter, lane, epi_tid, is_bf16, my,
-                                 t.n0 + (int)rank * 128, tok0, p.N, clip_out, t.t_end);
+          pair_store_tile_staged<MULTI>(staging, chunk_it, taddr, n_cols, quarter, lane, epi_tid, is_bf16, my,
+                                        t.n0 + (int)rank * 128, tok0, p.N, clip_out, t.t_end, p.alpha[0]);
         } else {
 #pragma unroll 1
           for (int c = 0; c < n_cols; c += 32) {

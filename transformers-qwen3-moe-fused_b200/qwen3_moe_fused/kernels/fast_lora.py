@@ -14,7 +14,8 @@ Differences in how the same quantities are computed:
     i.e. two thin grouped GEMMs per matrix, instead of a full (E, out, in) weight-gradient
     GEMM followed by two einsum projections (:139-149);
   * on dense 16-bit weights every `base product + s * (t B)` is one launch that contracts both operand
-    pairs into one accumulator (dx: four pairs), with s applied to the fp32 accumulator of the thin factor.
+    pairs into one accumulator (dx: four pairs), with s applied to fp32 accumulators: in bf16 to the thin factor's,
+    in fp16 (powers of two) to those of the products with the thin factor, which is held as it is.
 """
 import ctypes
 import math
@@ -40,11 +41,12 @@ def _dense(weight, quant_state, dtype):
 def _fits_fused(x, base, quant, adapters, scales, m_sizes) -> bool:
     """Whether the fused form takes the call: dense 16-bit base weights and adapters of matching shapes, ranks that are
     multiples of 8 (16-byte rows of the thin factors; gate and up side by side within the 256 columns of one tile), plain
-    numbers as factors.  In fp16 the factor moves onto the thin product, so it must not be able to push that out of
-    range: 1/16..16 is four of the format's 30 binades.  Everything else takes the general form below."""
+    numbers as factors.  In fp16 powers of two only, 2^-7..2^7: any other factor would have to go onto the thin factors,
+    whose small values it would take low bits from (|s| < 1) or whose large ones it would push out of range (|s| > 1).
+    Everything else takes the general form below."""
     if any(q is not None for q in quant) or not all(type(s) in (int, float) and math.isfinite(s) for s in scales):
         return False
-    if x.dtype == torch.float16 and not all(1 / 16 <= abs(s) <= 16 for s in scales):
+    if x.dtype == torch.float16 and not all(math.frexp(abs(s))[0] == 0.5 and 2.0 ** -7 <= abs(s) <= 2.0 ** 7 for s in scales):
         return False
     if not eligible(x, (*base, *adapters), m_sizes):
         return False
@@ -79,7 +81,7 @@ class FastLora(torch.autograd.Function):
         ctx.fused = _fits_fused(x, (Gq, Uq, Wq), (Gqs, Uqs, Wqs), (Ag, Bg, Au, Bu, Aw, Bw), (Sg, Su, Sw), m_sizes)
         if ctx.fused:
             M, H, (E, I) = x.shape[0], x.shape[1], Gq.shape[:2]
-            # t_gu, t_w: the thin factors s x A^T of the LoRA products, gate and up side by side
+            # t_gu, t_w: the thin factors of the LoRA products (s x A^T; fp16: +-x A^T), gate and up side by side
             e, g, h, t_gu, t_w, y = (torch.empty((M, n), device=x.device, dtype=dt)
                                      for n in (I, I, I, Ag.shape[1] + Au.shape[1], Aw.shape[1], H))
             w = _lora_weights((Gq, Uq, Wq), (Ag, Au, Aw), (Bg, Bu, Bw), (Sg, Su, Sw))
