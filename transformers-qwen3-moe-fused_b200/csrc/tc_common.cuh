@@ -5,6 +5,7 @@
 #include <cuda.h>  // CUtensorMap (types only; the driver entry point is fetched at run time)
 
 #include "common.cuh"
+#include "tile_draw.cuh"
 
 namespace moe {
 namespace tc {
@@ -12,7 +13,9 @@ namespace tc {
 // ---------------------------------------------------------------------------------------
 // Bounded waiting.  A wait that exceeds WAIT_LIMIT_NS records `code` in the library's
 // device-side error word, raises the CTA-wide abort flag in shared memory and returns
-// false; every role then leaves its loops and the CTA runs its normal teardown.
+// false; every role then leaves its loops and the CTA runs its normal teardown.  A kernel whose grid
+// has more clusters than run at once claims the ones that have not started (tile_draw.cuh), so that
+// the launch as a whole ends after one such limit.
 // ---------------------------------------------------------------------------------------
 constexpr unsigned long long WAIT_LIMIT_NS = 2000000000ull;  // 2 s
 
@@ -71,6 +74,15 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volati
       }
     }
   }
+}
+
+// For what has to be waited for even after another role aborted (a copy on its way to this CTA's shared memory): the time
+// limit is the only reason to give up.
+__device__ __forceinline__ bool mbar_wait_through(uint64_t* bar, uint32_t parity) {
+  const unsigned long long t0 = global_ns();
+  while (!mbar_try_wait(bar, parity))
+    if (global_ns() - t0 > WAIT_LIMIT_NS) return false;
+  return true;
 }
 
 // ---------------------------------------------------------------------------------------
@@ -251,6 +263,26 @@ __device__ __forceinline__ int cluster_cancelled_cta(const void* response) {
       : "=&r"(x) : "r"(smem_u32(response)) : "memory");
   return x;
 }
+// The drawing thread's end of it, as tile_draw.cuh wants it: `bar` counts one arrival, `response` is 16 bytes.
+struct CancelPort {
+  uint64_t* bar;
+  uint4* response;
+  volatile int* abort_flag;
+  int code;  // recorded when wait() runs into its limit
+  uint32_t ph = 0;
+  __device__ __forceinline__ void request() {
+    mbar_expect_tx(bar, 16);
+    cluster_try_cancel(response, bar);
+  }
+  __device__ __forceinline__ bool wait() { return mbar_wait(bar, ph, abort_flag, code); }
+  __device__ __forceinline__ bool wait_through() { return mbar_wait_through(bar, ph); }
+  __device__ __forceinline__ int answer() {
+    ph ^= 1;
+    const int cta = cluster_cancelled_cta(response);
+    fence_proxy_async_smem();  // the response has been read before the next one may be written
+    return cta;
+  }
+};
 // Four rows of a 2-D tensor, given by their row indices, into four consecutive 128-byte rows of shared
 // memory (the tensor map's box is {64 elements, 1 row}); completion as for the loads above.  Rows whose
 // index lies outside the tensor are filled with zeros.  Not multicast.

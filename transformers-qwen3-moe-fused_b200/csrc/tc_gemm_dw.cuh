@@ -172,8 +172,9 @@ dw_kernel(const __grid_constant__ DwMaps maps, const GemmParams p) {
       bool ok = true;
       // single-CTA form: this thread also draws the work items (it asks for the next one before the loads of an item
       // and looks at the answer after them)
+      CancelPort port{&ctl->cancel_bar, &ctl->cancel_response, abort_flag, PW_CANCEL};
+      ClusterDraw<CancelPort> draw(port);
       int next = (int)blockIdx.x;
-      uint32_t draw_ph = 0;
       while (ok) {
         int item;
         if constexpr (PAIR) {
@@ -181,10 +182,7 @@ dw_kernel(const __grid_constant__ DwMaps maps, const GemmParams p) {
         } else {
           item = next;
           if (!feed.publish(item)) break;
-          if (item >= 0) {
-            mbar_expect_tx(&ctl->cancel_bar, 16);
-            cluster_try_cancel(&ctl->cancel_response, &ctl->cancel_bar);
-          }
+          if (item >= 0) draw.ask();
         }
         if (item < 0) break;
         const int e = sorted[item / per_expert];
@@ -238,12 +236,11 @@ dw_kernel(const __grid_constant__ DwMaps maps, const GemmParams p) {
         }
         if constexpr (!PAIR) {
           if (!ok) break;
-          if (!mbar_wait(&ctl->cancel_bar, draw_ph, abort_flag, PW_CANCEL)) break;
-          draw_ph ^= 1;
-          next = cluster_cancelled_cta(&ctl->cancel_response);
-          fence_proxy_async_smem();  // the response has been read before the next one may be written
+          next = draw.collect();
+          if (next == ClusterDraw<CancelPort>::ABANDONED) break;
         }
       }
+      if constexpr (!PAIR) draw.leave();
     }
   } else if (warp == 1) {
     // ------------------------------ MMA issuer (leader CTA) ------------------------------

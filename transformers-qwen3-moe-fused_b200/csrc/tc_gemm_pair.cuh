@@ -291,21 +291,10 @@ struct TileFeed {
     ++n;
     return true;
   }
-  // Body of the drawing thread when it has nothing else to do (NCTA = 2): the tiles of the clusters that have not
-  // started yet, after this cluster's own tile `first`; ids from `total` on (the grid is an upper bound) are passed over.
+  // Body of the drawing thread when it has nothing else to do (NCTA = 2).
   __device__ __forceinline__ void run_cancel(uint64_t* bar, uint4* response, int total, int first) {
-    uint32_t ph = 0;
-    for (int tile = first;;) {
-      if (tile < total && !publish(tile)) return;
-      mbar_expect_tx(bar, 16);
-      cluster_try_cancel(response, bar);
-      if (!mbar_wait(bar, ph, abort_flag, PW_CANCEL)) return;
-      ph ^= 1;
-      const int cta = cluster_cancelled_cta(response);
-      fence_proxy_async_smem();  // the response has been read before the next one may be written
-      if (cta < 0) { publish(-1); return; }
-      tile = cta >> 1;
-    }
+    CancelPort port{bar, response, abort_flag, PW_CANCEL};
+    hand_out_tiles<NCTA>(port, total, first, [this](int tile) { return publish(tile); });
   }
   // a reader (one thread): next tile id, or -1 when there are no more (or the wait was abandoned)
   __device__ __forceinline__ int take() {
