@@ -76,3 +76,31 @@ def test_combine_backward_twice(cuda):
     ref = twice(torch.einsum("tkh,tk->th", d[0][inv].view(T, k, H), d[1]), *d)
     for a, b in zip(got, ref):  # fp32 sums of up to H * k products of products
         assert (a.cpu().double() - b).norm() <= 1e-5 * b.norm()
+
+
+@pytest.mark.parametrize("norm", [False, True])
+def test_batched_gradients(cuda, norm):
+    """Several gradients at once through the router, and through the combine where only its weights want one: each as if it
+    had come alone."""
+    from qwen3_moe_fused.kernels.routing import combine, softmax_topk_autograd
+
+    T, E, k, H = 5, 12, 3, 24
+    gen = torch.Generator(device=cuda).manual_seed(0)
+    logits = torch.randn(T, E, device=cuda, generator=gen).requires_grad_()
+    weights, _ = softmax_topk_autograd(logits, k, norm, torch.float32)
+    inv = torch.randperm(T * k, device=cuda, generator=gen)
+    y = torch.randn(T * k, H, device=cuda, generator=gen)
+    w = weights.detach().requires_grad_()
+    out = combine(y, torch.argsort(inv).to(torch.int32), inv.to(torch.int32), w)
+    v_weights = torch.randn(4, T, k, device=cuda, generator=gen)
+    v_out = torch.randn(4, T, H, device=cuda, generator=gen)
+
+    def pull(res, leaf):
+        return lambda v: torch.autograd.grad(res, leaf, v, retain_graph=True)[0]
+
+    got = [torch.autograd.grad(weights, logits, v_weights, is_grads_batched=True, retain_graph=True)[0],
+           torch.func.vmap(pull(weights, logits))(v_weights), torch.func.vmap(pull(out, w))(v_out)]
+    want = [torch.stack([pull(res, leaf)(v) for v in vs])
+            for res, leaf, vs in ((weights, logits, v_weights), (weights, logits, v_weights), (out, w, v_out))]
+    for a, b in zip(got, want):  # fp32 sums in another order
+        assert (a - b).norm() <= 1e-5 * b.norm()

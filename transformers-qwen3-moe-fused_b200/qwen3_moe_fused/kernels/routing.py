@@ -9,6 +9,12 @@ import torch
 from .. import _lib
 
 
+def _is_batched(t: torch.Tensor) -> bool:
+    """Whether `t` stands for several gradients at once (torch.func.vmap, or is_grads_batched of torch.autograd.grad).  Such a
+    tensor has no address for a kernel; ATen operations take it."""
+    return torch._C._functorch.is_batchedtensor(t) or torch._C._functorch.is_legacy_batchedtensor(t)
+
+
 @torch.no_grad()
 def softmax_topk(router_logits: torch.Tensor, k: int, norm_topk_prob: bool, out_dtype: torch.dtype):
     """(weights (T,k) out_dtype, experts (T,k) int64); winners ordered by probability
@@ -42,6 +48,14 @@ class SoftmaxTopk(torch.autograd.Function):
     @staticmethod
     def backward(ctx, dweights, _dexperts):
         logits, experts = ctx.saved_tensors
+        if _is_batched(dweights):
+            with torch.enable_grad():
+                lg = logits.detach().requires_grad_()
+                sel = torch.softmax(lg, dim=1, dtype=torch.float32).gather(1, experts)
+                if ctx.norm:
+                    sel = sel / sel.sum(dim=-1, keepdim=True)
+                (grad,) = torch.autograd.grad(sel.to(dweights.dtype), lg, dweights)
+            return grad, None, None, None
         T, E = logits.shape
         dweights = dweights.contiguous()
         grad = torch.empty_like(logits)
@@ -139,7 +153,7 @@ class Combine(torch.autograd.Function):
         T, k = weights.shape
         dout = dout.contiguous()
         dy = dw = None
-        if torch.is_grad_enabled():  # create_graph: operations that autograd can follow a second time
+        if torch.is_grad_enabled() or _is_batched(dout):  # (create_graph: operations that autograd can follow a second time)
             if ctx.needs_input_grad[0]:
                 dy = gather_rows(dout, sort_idx, inv_sort_idx, k) * weights.reshape(-1)[sort_idx.long()].unsqueeze(1)
             if ctx.needs_input_grad[3]:
