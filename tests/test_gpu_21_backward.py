@@ -103,3 +103,33 @@ def test_batched_gradients(cuda, norm):
     want = [torch.stack([pull(res, leaf)(v) for v in vs]) for res, leaf, vs in ((weights, logits, v_weights), (out, w, v_out))]
     for a, b in zip(got, want):  # fp32 sums in another order
         assert (a - b).norm() <= 1e-5 * b.norm()
+
+
+def test_hooks_that_change_layout_or_type(cuda):
+    """What saved-tensor hooks give back with other strides or in another type still gives the gradients it holds."""
+    from qwen3_moe_fused.kernels.routing import combine, softmax_topk_autograd
+
+    T, E, k, H = 5, 12, 3, 24
+    gen = torch.Generator(device=cuda).manual_seed(0)
+    logits = torch.randn(T, E, device=cuda, generator=gen).requires_grad_()
+    inv = torch.randperm(T * k, device=cuda, generator=gen)
+    sort_idx, inv = torch.argsort(inv).to(torch.int32), inv.to(torch.int32)
+    y = torch.randn(T * k, H, device=cuda, generator=gen).to(torch.bfloat16).requires_grad_()
+    dout = torch.randn(T, H, device=cuda, generator=gen).to(torch.bfloat16)
+
+    def grads():
+        weights, _ = softmax_topk_autograd(logits, k, True, torch.bfloat16)
+        return torch.autograd.grad(combine(y, sort_idx, inv, weights), (y, logits), dout)
+
+    def other_strides(t):
+        return t.mT.contiguous().mT if t.ndim == 2 else t
+
+    def other_type(t):
+        return t.float() if t.dtype == torch.bfloat16 else t
+
+    want = grads()
+    for change in (other_strides, other_type):
+        with torch.autograd.graph.saved_tensors_hooks(lambda t: t, change):
+            got = grads()
+        for a, b in zip(got, want):  # one rounding to bf16 on either side
+            assert (a.double() - b.double()).norm() <= 2.0 ** -7 * b.double().norm()

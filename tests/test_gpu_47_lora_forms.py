@@ -119,3 +119,33 @@ def test_which_form(cuda, fused, change):
         # chains of at most six roundings one after the other, each at most ROUND of what it applies to
         assert (g.double() - r).norm() <= 6 * ROUND[dtype] * r.norm()
     assert _lib.read_error_flag() == 0
+
+
+@pytest.mark.parametrize("which", ["hook", "moved base"])
+def test_backward_checks_what_it_reads(cuda, which):
+    """The backward in one accumulator per projection takes addresses: saved tensors that hooks gave back with other strides,
+    and base weights that left the device since the forward, are refused as in the general form."""
+    from qwen3_moe_fused.kernels.fast_lora import fast_lora
+
+    args, m_sizes, leaves = case(cuda)
+    if which == "hook":
+        with torch.autograd.graph.saved_tensors_hooks(lambda t: t, lambda t: t.mT.contiguous().mT):
+            y = fast_lora(*args, m_sizes)
+    else:
+        y = fast_lora(*args, m_sizes)
+        args[11].data = args[11].data.cpu()
+    assert y.grad_fn.fused
+    with pytest.raises(AssertionError):
+        torch.autograd.grad(y, leaves, torch.ones_like(y))
+
+
+def test_backward_with_saved_tensors_on_the_host(cuda):
+    """Saved on the host and brought back unchanged: the same bits."""
+    from qwen3_moe_fused.kernels.fast_lora import fast_lora
+
+    args, m_sizes, leaves = case(cuda)
+    dy = torch.randn_like(args[0])
+    want = torch.autograd.grad(fast_lora(*args, m_sizes), leaves, dy)
+    with torch.autograd.graph.save_on_cpu():
+        y = fast_lora(*args, m_sizes)
+    assert all(torch.equal(a, b) for a, b in zip(torch.autograd.grad(y, leaves, dy), want))

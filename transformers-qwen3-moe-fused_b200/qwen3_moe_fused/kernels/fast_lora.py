@@ -60,6 +60,12 @@ def _fits_fused(x, base, quant, adapters, scales, m_sizes) -> bool:
         Bg.shape == (E, I, rg) and Bu.shape == (E, I, ru) and Bw.shape == (E, H, rw)
 
 
+def _rows_fit(x, I, rg, ru, rw, e, g, t_gu, t_w) -> bool:
+    """Whether the intermediates are as the fused forward left them."""
+    return all(t.shape == (x.shape[0], n) and t.dtype == x.dtype and t.device == x.device and t.is_contiguous()
+               and t.data_ptr() % 16 == 0 for t, n in ((e, I), (g, I), (t_gu, rg + ru), (t_w, rw)))
+
+
 def _lora_weights(base, a, b, scales) -> _lib.LoraWeights:
     ptrs = lambda ts: (ctypes.c_void_p * 3)(*(t.data_ptr() for t in ts))
     return _lib.LoraWeights(ptrs(base), ptrs(a), ptrs(b), (ctypes.c_float * 3)(*scales), (ctypes.c_int * 3)(*(t.shape[1] for t in a)))
@@ -117,10 +123,14 @@ class FastLora(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, dy):
-        if ctx.fused and _lib.load().moe_get_gemm_path() == _lib.PATH_AUTO:  # (may have been switched since the forward)
-            return FastLora._backward_fused(ctx, dy)
         Gq, Gqs, Sg, Uq, Uqs, Su, Wq, Wqs, Sw, m_sizes = ctx.custom_saved_tensors
-        x, Ag, Bg, Au, Bu, Aw, Bw, e, g = ctx.saved_tensors[:9]
+        saved = ctx.saved_tensors
+        x, Ag, Bg, Au, Bu, Aw, Bw, e, g = saved[:9]
+        # (since the forward the GEMM path may have been switched, base weights moved, saved tensors changed by hooks: the
+        # fused form takes addresses, the general form's launchers check each operand)
+        if ctx.fused and _fits_fused(x, (Gq, Uq, Wq), (Gqs, Uqs, Wqs), (Ag, Bg, Au, Bu, Aw, Bw), (Sg, Su, Sw), m_sizes) and \
+                _rows_fit(x, Gq.shape[1], Ag.shape[1], Au.shape[1], Aw.shape[1], *saved[7:]):
+            return FastLora._backward_fused(ctx, dy, saved)
         dt = x.dtype
         dy = dy.contiguous().to(dt)
 
@@ -169,9 +179,9 @@ class FastLora(torch.autograd.Function):
 
 
     @staticmethod
-    def _backward_fused(ctx, dy):
+    def _backward_fused(ctx, dy, saved):
         Gq, _, Sg, Uq, _, Su, Wq, _, Sw, m_sizes = ctx.custom_saved_tensors
-        x, Ag, Bg, Au, Bu, Aw, Bw, e, g, t_gu, t_w = ctx.saved_tensors
+        x, Ag, Bg, Au, Bu, Aw, Bw, e, g, t_gu, t_w = saved
         dy = dy.contiguous().to(x.dtype)
         if dy.data_ptr() % 16:
             dy = dy.clone()

@@ -15,6 +15,11 @@ def _is_batched(t: torch.Tensor) -> bool:
     return torch._C._functorch.is_batchedtensor(t) or torch._C._functorch.is_legacy_batchedtensor(t)
 
 
+def _addressable(like: torch.Tensor, *tensors: torch.Tensor) -> bool:
+    """Whether a kernel may read these next to `like`: saved-tensor hooks may have given back another device or layout."""
+    return all(t.device == like.device and t.is_contiguous() for t in tensors)
+
+
 @torch.no_grad()
 def softmax_topk(router_logits: torch.Tensor, k: int, norm_topk_prob: bool, out_dtype: torch.dtype):
     """(weights (T,k) out_dtype, experts (T,k) int64); winners ordered by probability
@@ -48,7 +53,7 @@ class SoftmaxTopk(torch.autograd.Function):
     @staticmethod
     def backward(ctx, dweights, _dexperts):
         logits, experts = ctx.saved_tensors
-        if _is_batched(dweights):
+        if _is_batched(dweights) or not _addressable(dweights, logits, experts) or experts.dtype != torch.int64:
             with torch.enable_grad():
                 lg = logits.detach().requires_grad_()
                 sel = torch.softmax(lg, dim=1, dtype=torch.float32).gather(1, experts)
@@ -153,7 +158,9 @@ class Combine(torch.autograd.Function):
         T, k = weights.shape
         dout = dout.contiguous()
         dy = dw = None
-        if torch.is_grad_enabled() or _is_batched(dout):  # (create_graph: operations that autograd can follow a second time)
+        # create_graph wants operations that autograd can follow a second time
+        if torch.is_grad_enabled() or _is_batched(dout) or not _addressable(dout, y, sort_idx, inv_sort_idx, weights) or \
+                not y.dtype == weights.dtype == dout.dtype or inv_sort_idx.dtype != torch.int32:
             if ctx.needs_input_grad[0]:
                 dy = gather_rows(dout, sort_idx, inv_sort_idx, k) * weights.reshape(-1)[sort_idx.long()].unsqueeze(1)
             if ctx.needs_input_grad[3]:
