@@ -60,10 +60,15 @@ def _fits_fused(x, base, quant, adapters, scales, m_sizes) -> bool:
         Bg.shape == (E, I, rg) and Bu.shape == (E, I, ru) and Bw.shape == (E, H, rw)
 
 
-def _rows_fit(x, I, rg, ru, rw, e, g, t_gu, t_w) -> bool:
-    """Whether the intermediates are as the fused forward left them."""
-    return all(t.shape == (x.shape[0], n) and t.dtype == x.dtype and t.device == x.device and t.is_contiguous()
-               and t.data_ptr() % 16 == 0 for t, n in ((e, I), (g, I), (t_gu, rg + ru), (t_w, rw)))
+def _still_fits(tensors, shapes, m_sizes) -> bool:
+    """Whether what the fused form took or made in the forward can still be read by address: `shapes` as they were, one type
+    and device, 16-byte aligned and contiguous, the GEMM path not switched."""
+    dtype, device = tensors[0].dtype, tensors[0].get_device()
+    for t, shape in zip(tensors, shapes):
+        if t.shape != shape or t.dtype != dtype or t.get_device() != device or not t.is_contiguous() or t.data_ptr() % 16:
+            return False
+    return device >= 0 and m_sizes.get_device() == device and m_sizes.is_contiguous() and m_sizes.numel() == shapes[-1][0] and \
+        _lib.load().moe_get_gemm_path() == _lib.PATH_AUTO
 
 
 def _lora_weights(base, a, b, scales) -> _lib.LoraWeights:
@@ -99,7 +104,9 @@ class FastLora(torch.autograd.Function):
                     _lib.stream_ptr(x.device))
             _lib.check(status, "moe_lora_mlp_fwd")
             ctx.custom_saved_tensors = (Gq, Gqs, Sg, Uq, Uqs, Su, Wq, Wqs, Sw, m_sizes)
-            ctx.save_for_backward(x, Ag, Bg, Au, Bu, Aw, Bw, e, g, t_gu, t_w)
+            saved = (x, Ag, Bg, Au, Bu, Aw, Bw, e, g, t_gu, t_w)
+            ctx.save_for_backward(*saved)
+            ctx.shapes = [t.shape for t in (*saved, Gq, Uq, Wq)]
             return y
 
         def base(_x, _wq, _wqs):
@@ -128,8 +135,7 @@ class FastLora(torch.autograd.Function):
         x, Ag, Bg, Au, Bu, Aw, Bw, e, g = saved[:9]
         # (since the forward the GEMM path may have been switched, base weights moved, saved tensors changed by hooks: the
         # fused form takes addresses, the general form's launchers check each operand)
-        if ctx.fused and _fits_fused(x, (Gq, Uq, Wq), (Gqs, Uqs, Wqs), (Ag, Bg, Au, Bu, Aw, Bw), (Sg, Su, Sw), m_sizes) and \
-                _rows_fit(x, Gq.shape[1], Ag.shape[1], Au.shape[1], Aw.shape[1], *saved[7:]):
+        if ctx.fused and _still_fits((*saved, Gq, Uq, Wq), ctx.shapes, m_sizes):
             return FastLora._backward_fused(ctx, dy, saved)
         dt = x.dtype
         dy = dy.contiguous().to(dt)
