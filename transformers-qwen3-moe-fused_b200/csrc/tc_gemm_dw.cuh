@@ -5,8 +5,8 @@
 // follows them in memory belongs to the next expert: its MMA steps of 16 rows must find zeros there (in both operands,
 // an infinity times zero would not do).  TMA brings whole groups of 16 rows in one box, and the last, partial group as
 // boxes of 8, 4, 2 and 1 rows that end exactly at the expert's last row; the rest of the group is filled by boxes that
-// start past the tensor's last row, which TMA fills with zeros.  At most five boxes per operand chunk and expert, on maps
-// that do not depend on the groups.  (Per-expert maps whose row extent ends at the group did the same before: a launch of
+// start past the tensor's last row, which TMA fills with zeros.  At most eight boxes per operand chunk of an expert's last
+// block (63 rows: three whole groups, five in the partial one), on maps that do not depend on the groups.  (Per-expert maps whose row extent ends at the group did the same before: a launch of
 // its own in front of each GEMM, 5.5 us and a gap, with the same time in the GEMM.  Forward + dX + dW: 294 -> 286 us at
 // 5003 rows 2048 -> 768, 1036 -> 1021 us at 65536 rows 2048 -> 1536.)
 //
@@ -221,16 +221,15 @@ dw_kernel(const __grid_constant__ DwMaps maps, const GemmParams p) {
             if (tail) {
               // halve the group down to the boundary: real rows before it, rows past the tensor (zeros) behind it
               const int base = left & ~15;
-              int lo = 0, hi = 16;  // the boundary lies in (lo, hi]
-              for (int box = 2; box < DW_BOXES && tail > lo && tail < hi; ++box) {
+              int lo = 0, hi = 16;  // the boundary lies in [lo, hi)
+              for (int box = 2; box < DW_BOXES && tail > lo; ++box) {
                 const int mid = lo + dw_box_rows(box);
                 if (tail >= mid) { load_rows(box, base + lo, row + base + lo); lo = mid; }
                 else { load_rows(box, base + mid, (int)p.M); hi = mid; }
               }
-              // [lo, hi) is all real (tail == hi) or all behind the boundary (tail == lo); its size is a box's
+              // tail == lo now: [lo, hi) lies behind the boundary; its size is a box's
               const int rest = hi - lo;
-              const int box = rest == 8 ? 2 : rest == 4 ? 3 : rest == 2 ? 4 : 5;
-              if (rest > 0) load_rows(box, base + lo, tail == hi ? row + base + lo : (int)p.M);
+              load_rows(rest == 8 ? 2 : rest == 4 ? 3 : rest == 2 ? 4 : 5, base + lo, (int)p.M);
             }
           }
         }
