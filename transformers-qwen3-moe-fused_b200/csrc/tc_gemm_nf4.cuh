@@ -4,8 +4,8 @@
 // Same tiling as pair_fwd_kernel<false> (accumulator rows = 256 weight rows of one expert,
 // 128 per CTA; accumulator columns = up to 256 tokens; two TMEM accumulators so the epilogue
 // overlaps the next tile), but the weight half-tile of a stage is not loaded as 16-bit data:
-// TMA brings the 4 KB of packed 4-bit codes (128 rows x 32 bytes) and twenty decode warps per
-// CTA (five groups of four, taking k-blocks in turn) expand them to the swizzled K-major 16-bit tile the MMA reads.  HBM and L2 see
+// TMA brings the 4 KB of packed 4-bit codes (128 rows x 32 bytes) and sixteen decode warps per
+// CTA (four groups of four, taking k-blocks in turn) expand them to the swizzled K-major 16-bit tile the MMA reads.  HBM and L2 see
 // 0.5 + 4/blocksize bytes per weight instead of 2.
 //
 // Synchronisation per stage s:
@@ -13,8 +13,8 @@
 //   full[s]   (leader)  token tiles of both CTAs have landed            TMA tx from both CTAs
 //   ready[s]  (leader)  decoded weight tiles of both CTAs are written   8 arrivals (4 warps x 2 CTAs)
 //   empty[s]  (both)    the MMAs that read the stage have completed     tcgen05.commit, multicast
-// The decode warps publish their shared-memory writes to the async proxy
-// (fence.proxy.async) before arriving on the leader's barrier.
+// The decode warps publish their shared-memory writes to the async proxy (fence.proxy.async) and, at cluster scope, to
+// the leader's MMA thread before arriving on its barrier.
 //
 // pair_fwd_nf4_kernel<IS_BF16, true> is the transposed form (dX through an NF4 weight):
 //   y[t, n] = sum_k w[e, k, n] x[t, k],  w = the (E, K, N) NF4 tensor, n contiguous in a block
@@ -36,13 +36,15 @@ namespace moe {
 namespace tc {
 
 constexpr int NF4P_STAGES = 5;
-constexpr int NF4P_GROUPS = 5;                                  // decode groups of four warps, taking k-blocks in turn
+constexpr int NF4P_GROUPS = 4;                                  // decode groups of four warps, taking k-blocks in turn
 constexpr int NF4P_THREADS = 192 + NF4P_GROUPS * 128;           // TMA, MMA, 4 epilogue warps + the decode warps
-// A decode group must meet the phases of a stage's qfull barrier one after the other.  If it came back to a
-// stage after skipping a phase (say 4 groups on 5 stages: k-block j, then j + 4 in the stage of j - 1), it
-// could test for the phase of j + 4 while the codes of j - 1 were still on their way (loads complete in any
-// order); the parity of that phase equals the one before j - 1, so the test would pass at once.
-static_assert(NF4P_STAGES % NF4P_GROUPS == 0, "every stage belongs to one decode group");
+// A decode group comes back to a stage after skipping phases of its barriers: from k-block j - 4 it goes to j, in
+// the stage of j - 5, whose codes may still be on their way (loads complete in any order).  The phase of j has the
+// parity of the one before that of j - 5, so a test of qfull alone would pass at once.  The group therefore waits until
+// j - 5 has been consumed (empty) first, which no test can mistake: it has seen the codes of j - 4, for which the
+// producer had to wait until j - 10 was consumed, and j itself cannot be consumed without the group.  The codes of
+// j - 5 have then landed, and those of j + 5 cannot be asked for yet.
+static_assert(NF4P_GROUPS < NF4P_STAGES, "a group's first k-block is the first of its stage; j - groups is loaded after j - stages");
 constexpr int NF4P_PACKED_BYTES = 128 * (BK / 2);               // 4 KB
 constexpr int NF4P_STAGE_BYTES = 2 * PAIR_HALF_BYTES + NF4P_PACKED_BYTES;  // 36 KB
 
@@ -280,8 +282,9 @@ pair_fwd_nf4_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
     // ------------------------------ decode warps (both CTAs) ------------------------------
     // NF4P_GROUPS groups of four warps take the k-blocks in turn, so the decode of one k-block (a
     // few hundred cycles of dependent work per thread) overlaps the decode of the next ones.
-    // Measured at 262144 rows: 2 groups 1162 TFLOP/s, 4 groups 1255 (5: see the static_assert above).  Inside a
-    // group, thread -> weight row (t % 128) of this CTA's half-tile; it decodes the row's 64
+    // Measured at (128, 1536, 2048), forward, 4096 / 32768 / 131072 rows: 4 groups (no spills) 169 / 202 / 679 us, 5 groups
+    // (72 registers, no spills) 171 / 208 / 687; with an arrival that releases everything at cluster scope, 204 / 235 / 798:
+    // it waited for the absmax loads that are kept in flight.  Inside a group, thread -> weight row (t % 128) of this CTA's half-tile; it decodes the row's 64
     // weights of the k-block (32 packed bytes, one absmax).
     const int t = threadIdx.x - 6 * 32;
     const int row = t & 127;
@@ -325,6 +328,7 @@ pair_fwd_nf4_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
           const int kbn = kb + NF4P_GROUPS * AM_AHEAD;
           am_ring[AM_AHEAD - 1] = (n_ok && kbn < k_blocks) ? __ldg(q.absmax + ((row_flat + (int64_t)kbn * kb_stride) >> q.shift)) : 0.f;
         }
+        if (my_it >= STAGES && !mbar_wait(&ctl->empty[s], ph ^ 1, abort_flag, PW_EMPTY)) { ok = false; break; }
         if (!mbar_wait(&ctl->qfull[s], ph, abort_flag, PW_FULL)) { ok = false; break; }
         uint8_t* st = smem + s * STAGE_BYTES;
         // forward: 128 rows x 32 bytes; transposed: 64 rows x 64 bytes, this thread's half of its row
@@ -342,7 +346,7 @@ pair_fwd_nf4_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
         }
         fence_proxy_async_smem();
         __syncwarp();
-        if (lane == 0) mbar_arrive_release_cluster(ready_leader0 + s * 8);
+        if (lane == 0) mbar_arrive_release_own_smem_cluster(ready_leader0 + s * 8);
       }
       it += k_blocks;
     }
